@@ -1,0 +1,405 @@
+// Lightmap::blur (Lightmap.cpp:196-220): a 3x3 mean over the valid lumels of
+// each interior texel's window, in place and in scan order, so that texel
+// (x, y) reads the already-blurred (x-1..x+1, y-1) and (x-1, y) and the
+// original rest of its window.  Sums run in the reference's window order;
+// the result is the reference's, bit for bit.
+//
+// What bounds it: the chain.  Texel (x, y) needs (x-1, y) and (x+1, y-1), so
+// a W x H map has W + 2 H dependent steps of six additions, one product and
+// a lane shuffle however many units work on it; memory (32 bytes a texel)
+// takes a twentieth of that.  So what is not in the chain is kept out of it:
+//
+//   k_blur_skew  lays the colours out as the chain reads them: bands of 32
+//                rows, one lane per row, lane l two columns behind lane l-1,
+//                planar, zero where the texel is not valid, with the
+//                window's 1 / count beside them (coalesced loads, no flag
+//                tests, no divisions in the chain).
+//   k_blur_wave  one cluster of eight CTAs; a warp carries one colour channel
+//                of one band, so three warps work on a band and sixteen bands
+//                are in flight (about thirteen are busy at 1024 columns).
+//                The row above comes from the neighbouring lane by a shuffle;
+//                from the band above, eight columns at a time, through an
+//                inbox in shared memory that the band above fills with
+//                st.async (the mbarrier that counts its bytes orders it: no
+//                fence stands in the chain).
+//
+//   k_blur_unskew  takes the blurred values back to the map.
+//
+// Measured: 1024 x 1024 9.4 ms as one block with a barrier per step (3,066
+// steps of about 3 us), 0.30 ms as here; 128 x 128 0.19 -> 0.05 ms.  A step
+// of the wave takes about 75 ns.  Lanes three columns apart take the shuffle
+// out of the chain (63 ns a step) but need more steps: 0.34 ms.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdarg>
+#include <cstdint>
+#include <cstdio>
+
+#include "../../include/relight_b200.h"
+#include "rl_device.cuh"
+
+int rl_internal_fail(int code, const char* msg);
+int rl_internal_pool_alloc(void** p, size_t bytes, cudaStream_t st);
+
+namespace {
+
+constexpr int kRows = 32;        // rows per band, one per lane
+constexpr int kLag = 2;          // columns between neighbouring lanes
+constexpr int kGroup = 8;        // inbox columns per mbarrier phase
+constexpr int kCtas = 8;         // the cluster
+constexpr int kBandsPerCta = 2;
+constexpr int kStages = 4;       // ring of groups of steps whose colours are read ahead (about 1,500 clocks)
+constexpr int kStageFloats = 2 * kGroup * kRows + 16;  // own-row colours, reciprocal counts, the row below the last lane
+constexpr int kSlots = kCtas * kBandsPerCta;
+constexpr int kThreads = kBandsPerCta * 3 * 32;
+constexpr int kSkewCols = 32;    // columns of the skewed layout per k_blur_skew block
+// The last lane's first step of a group is column -kLag (kRows - 1) mod kGroup: its inbox groups, which hold column x
+// at position x + kGroup - 1, start kShift values before its groups of steps.
+constexpr int kShift = (kGroup * kRows + kGroup - 1 - kLag * (kRows - 1)) % kGroup;
+constexpr int kHist = kShift > kLag ? kShift : kLag;
+constexpr uint32_t kSpin = 1u << 19;  // bounded waits (about a second)
+
+__host__ __device__ inline int blur_groups(int W) { return (W + kGroup - 2) / kGroup + 1; }
+// Steps of one band: until the last lane has completed the last inbox group (then it is past column W - 1); whole
+// groups.
+__host__ __device__ inline int blur_steps(int W) {
+    const int steps = kGroup * blur_groups(W) + kLag * (kRows - 1) - (kGroup - 1) + kShift;
+    return (steps + 2 * kGroup - 1) / (2 * kGroup) * (2 * kGroup);
+}
+// One warp's shared memory: the read-ahead ring, its inbox (a whole row, so that no sender ever waits for room), then
+// a barrier per group.
+__host__ __device__ inline uint32_t blur_part(int W) {
+    return kStages * kStageFloats * 4 + (uint32_t)blur_groups(W) * kGroup * 4 + ((uint32_t)blur_groups(W) * 8 + 15) / 16 * 16;
+}
+
+// The skewed planes: o[c][band][t][lane] = colour c of (x + 1, y) where valid, else 0, and o[3] = 1 / count of the
+// window of (x, y), negative where (x, y) itself is not valid and 0 where it is not written (no valid lumel in the
+// window, border, outside), for x = t - kLag lane, y = 1 + 32 band + lane.  e[c][band][t] is the colour of
+// (x + 1, y + 1) for the band's last lane.
+struct Skew {
+    float* o;
+    float* e;
+    int bands, steps;
+    __host__ __device__ size_t plane() const { return (size_t)bands * steps * kRows; }
+};
+
+__device__ __forceinline__ float masked(const rl::DevMap& m, int x, int y, int c) {
+    if (x < 0 || x >= m.width || y < 0 || y >= m.height) return 0.f;
+    const size_t i = (size_t)y * m.width + x;
+    return (m.flags[i] & 1) ? m.color[3 * i + c] : 0.f;
+}
+
+// Rows are read along x and written along the lanes, through shared memory.
+__global__ void __launch_bounds__(256) k_blur_skew(rl::DevMap m, Skew s) {
+    __shared__ float tile[4][kSkewCols][kRows + 1];
+    const int W = m.width, H = m.height;
+    const int band = blockIdx.y, t0 = blockIdx.x * kSkewCols;
+    const int col = threadIdx.x & 31;
+    for (int l = threadIdx.x >> 5; l < kRows; l += 8) {
+        const int x = t0 + col - kLag * l, y = 1 + kRows * band + l;
+        float inv = 0.f, c[3] = {0.f, 0.f, 0.f};
+        if (y < H && x >= -1 && x + 1 < W) {  // row H - 1 too: it lies below the last blurred row
+            const size_t i = (size_t)y * W + x + 1;
+            if (m.flags[i] & 1) {
+                c[0] = m.color[3 * i];
+                c[1] = m.color[3 * i + 1];
+                c[2] = m.color[3 * i + 2];
+            }
+        }
+        if (y <= H - 2 && x >= 1 && x <= W - 2) {
+            int count = 0;
+            for (int dy = -1; dy <= 1; dy++)
+                for (int dx = -1; dx <= 1; dx++) count += m.flags[(size_t)(y + dy) * W + x + dx] & 1;
+            if (count) inv = 1.0f / (float)count;
+            if (!(m.flags[(size_t)y * W + x] & 1)) inv = -inv;
+        }
+        for (int k = 0; k < 3; k++) tile[k][col][l] = c[k];
+        tile[3][col][l] = inv;
+    }
+    __syncthreads();
+    const size_t base = ((size_t)band * s.steps + t0) * kRows, plane = s.plane();
+    const int n = min(kSkewCols, s.steps - t0) * kRows;
+    for (int q = threadIdx.x; q < n; q += 256)
+        for (int k = 0; k < 4; k++) s.o[k * plane + base + q] = tile[k][q / kRows][q % kRows];
+    if (threadIdx.x < min(kSkewCols, s.steps - t0)) {
+        const int t = t0 + threadIdx.x;
+        for (int k = 0; k < 3; k++)
+            s.e[((size_t)k * s.bands + band) * s.steps + t] =
+                masked(m, t - kLag * (kRows - 1) + 1, 1 + kRows * (band + 1), k);
+    }
+}
+
+// The blurred values back to the map, where one was written.
+__global__ void __launch_bounds__(256) k_blur_unskew(rl::DevMap m, Skew s) {
+    __shared__ float tile[4][kSkewCols][kRows + 1];
+    const int band = blockIdx.y, t0 = blockIdx.x * kSkewCols;
+    const size_t base = ((size_t)band * s.steps + t0) * kRows, plane = s.plane();
+    const int n = min(kSkewCols, s.steps - t0) * kRows;
+    for (int q = threadIdx.x; q < n; q += 256)
+        for (int k = 0; k < 4; k++) tile[k][q / kRows][q % kRows] = s.o[k * plane + base + q];
+    __syncthreads();
+    const int col = threadIdx.x & 31;
+    if (t0 + col >= s.steps) return;
+    for (int l = threadIdx.x >> 5; l < kRows; l += 8) {
+        if (tile[3][col][l] == 0.f) continue;
+        const int x = t0 + col - kLag * l, y = 1 + kRows * band + l;
+        float* o = m.color + 3 * ((size_t)y * m.width + x);
+        for (int k = 0; k < 3; k++) o[k] = tile[k][col][l];
+    }
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cta_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t peer_addr(uint32_t local, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// Where `on`, store eight floats at a (remote) 16-byte aligned shared address and count their bytes on its barrier.
+__device__ __forceinline__ void send8(bool on, uint32_t addr, const float (&v)[8], uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %10, 0;\n\t"
+        "@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%9];\n\t"
+        "@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%1], {%6, %7, %8, %11}, [%9];\n\t}" ::"r"(
+            addr),
+        "r"(addr + 16), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+        "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])),
+        "r"(bar), "r"((uint32_t)on), "r"(__float_as_uint(v[7]))
+        : "memory");
+}
+__device__ __forceinline__ void expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kSpin; i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void copy16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// One group of steps' inputs: own-row colours kLag + 1 columns ahead, reciprocal counts, the last lane's row below.
+struct Inputs {
+    float o[kGroup], inv[kGroup], e[kGroup];
+    __device__ __forceinline__ void load(const float* stage, int lane) {
+#pragma unroll
+        for (int u = 0; u < kGroup; u++) {
+            o[u] = stage[u * kRows + lane];
+            inv[u] = stage[(kGroup + u) * kRows + lane];
+        }
+        const float4* pe = reinterpret_cast<const float4*>(stage + 2 * kGroup * kRows);
+        const float4 a = pe[0], b = pe[1];
+        e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w;
+        e[4] = b.x; e[5] = b.y; e[6] = b.z; e[7] = b.w;
+    }
+};
+
+// The rows of band b are 1 + 32 b + lane.  grid = one cluster.
+__global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1)
+    k_blur_wave(rl::DevMap m, Skew s, int* err) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int W = m.width, H = m.height;
+    const int groups = blur_groups(W), cols = groups * kGroup;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cta_rank();
+    const int slot = (int)rank * kBandsPerCta + warp / 3, ch = warp % 3;
+    const uint32_t part = blur_part(W);
+    float* ring = reinterpret_cast<float*>(smem + warp * part);
+    float* inbox = ring + kStages * kStageFloats;
+    const uint32_t bars = smem_addr(inbox + cols);
+    for (int g = lane; g < groups; g += 32)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * g) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int g = lane; g < groups; g += 32) expect(bars + 8 * g, 4 * kGroup);
+    if (slot == 0)  // the row above the first band is the map's border
+        for (int p = lane; p < cols; p += 32) inbox[p] = masked(m, p - (kGroup - 1), 0, ch);
+    __syncwarp();
+    cluster_sync();
+    // the next slot's inbox and barriers
+    const int ns = (slot + 1) % kSlots;
+    const uint32_t nwarp = (uint32_t)((ns % kBandsPerCta) * 3 + ch);
+    const uint32_t next_box =
+        peer_addr(smem_addr(smem + nwarp * part) + kStages * kStageFloats * 4, (uint32_t)(ns / kBandsPerCta));
+    const uint32_t next_bar = next_box + (uint32_t)cols * 4;
+    bool dead = false;
+    int round = 0;
+    for (int band = slot; band < s.bands; band += kSlots, round++) {
+        const int y = 1 + kRows * band + lane;
+        const size_t plane = s.plane(), at = (size_t)band * s.steps * kRows + lane;
+        float* po = s.o + ch * plane + at;
+        const float* pi = s.o + 3 * plane + at;
+        const float* pe = s.e + ((size_t)ch * s.bands + band) * s.steps;
+        const uint32_t parity = (uint32_t)((slot == 0 ? round - 1 : round) & 1);
+        const bool sends = lane == kRows - 1 && band + 1 < s.bands;
+        // group g of the row above
+        float in[kGroup];
+        auto receive = [&](int g) {
+            if (g >= groups) return;
+            const uint32_t bar = bars + 8 * g;
+            if (band > 0 && !dead) dead = !__all_sync(0xffffffffu, wait_phase(bar, parity));
+            const float4 a = *reinterpret_cast<const float4*>(inbox + kGroup * g);
+            const float4 b = *reinterpret_cast<const float4*>(inbox + kGroup * g + 4);
+            in[0] = a.x; in[1] = a.y; in[2] = a.z; in[3] = a.w;
+            in[4] = b.x; in[5] = b.y; in[6] = b.z; in[7] = b.w;
+            __syncwarp();
+            // the next round's bytes; a barrier whose wait ran out is still armed
+            if (band > 0 && !dead && lane == 0) expect(bar, 4 * kGroup);
+        };
+        receive(0);
+        // sliding window: blurred (x-1, y-1), (x, y-1); blurred (x-1, y), original (x, y); original (x-1, y+1),
+        // (x, y+1).  Column 0 is lane 0's first; the others run up to theirs.
+        const bool first = lane == 0 && y <= H - 2;
+        float a1 = 0.f, a2 = lane == 0 ? in[kGroup - 1] : 0.f;
+        float b1 = 0.f, b2 = first ? masked(m, 0, y, ch) : 0.f;
+        float c1 = 0.f, c2 = first ? masked(m, 0, y + 1, ch) : 0.f;
+        float own[kLag];      // original (x + 1 .. x + kLag, y): the row-below shuffle reads the row kLag steps ahead
+        float hist[kHist];    // the latest blurred values, newest last
+#pragma unroll
+        for (int k = 0; k < kLag; k++) own[k] = po[k * kRows];
+#pragma unroll
+        for (int k = 0; k < kHist; k++) hist[k] = 0.f;
+        // The ring is filled by asynchronous copies, not by loads into registers: those wait in groups (a load's
+        // scoreboard is shared with later ones), which cost a full L2 latency every group.
+        auto fetch = [&](int t) {
+            float* stage = ring + (t / kGroup) % kStages * kStageFloats;
+            if (t < s.steps) {
+                // o is read kLag steps ahead; the band's plane ends kLag steps
+                // before the last group's reads (columns past W - 1) do
+                const int left = s.steps - t - kLag;
+                const float* so = po - lane + (size_t)(t + kLag) * kRows + 4 * lane;
+                const float* si = pi - lane + (size_t)t * kRows + 4 * lane;
+                if (lane / 8 < left) copy16(stage + 4 * lane, so);
+                if (lane / 8 + 4 < left) copy16(stage + 128 + 4 * lane, so + 128);
+                copy16(stage + 256 + 4 * lane, si);
+                copy16(stage + 384 + 4 * lane, si + 128);
+                if (lane < 2) copy16(stage + 512 + 4 * lane, pe + t + 4 * lane);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        // group t's inputs, once its copies (and those of kStages - 2 later groups at most) are outstanding
+        auto take = [&](Inputs& a, int t) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+            __syncwarp();
+            a.load(ring + (t / kGroup) % kStages * kStageFloats, lane);
+            __syncwarp();
+        };
+        auto group = [&](const Inputs& a, int t0) {
+            receive(t0 / kGroup + 1);
+            float c3[kGroup], v[kGroup], n[kHist + kGroup];
+#pragma unroll
+            for (int k = 0; k < kHist; k++) n[k] = hist[k];
+#pragma unroll
+            for (int u = 0; u < kGroup; u++) {
+                const float below = __shfl_down_sync(0xffffffffu, a.o[u], 1);
+                c3[u] = lane == kRows - 1 ? a.e[u] : below;
+            }
+            // the chain: nothing else stands in these eight steps
+#pragma unroll
+            for (int u = 0; u < kGroup; u++) {
+                const float above = __shfl_up_sync(0xffffffffu, n[kHist + u + 1 - kLag], 1);
+                const float a3 = lane == 0 ? in[u] : above;
+                const float b3 = u < kLag ? own[u % kLag] : a.o[u < kLag ? 0 : u - kLag];
+                float sum = 0.0f + a1;
+                sum += a2;
+                sum += a3;
+                sum += b1;
+                sum += b2;
+                sum += b3;
+                sum += c1;
+                sum += c2;
+                sum += c3[u];
+                v[u] = sum * fabsf(a.inv[u]);
+                b1 = n[kHist + u] = a.inv[u] > 0.f ? v[u] : b2;
+                a1 = a2; a2 = a3;
+                b2 = b3;
+                c1 = c2; c2 = c3[u];
+            }
+            // over the colours of these steps, which every reader has taken by now (one 128-byte line a step; written to
+            // the map from here, a step touches 32 lines, and six warps' stores took three times the chain)
+#pragma unroll
+            for (int u = 0; u < kGroup; u++) po[(size_t)(t0 + u) * kRows] = v[u];
+            // the inbox group that ends with this group's steps
+            float box[kGroup];
+#pragma unroll
+            for (int k = 0; k < kGroup; k++) box[k] = n[kHist - kShift + k];
+            const int g = (t0 - kLag * (kRows - 1) + kGroup - 1 - kShift) / kGroup;
+            send8(sends && t0 >= kLag * (kRows - 1) - (kGroup - 1) + kShift && g < groups,
+                  next_box + 4u * kGroup * (uint32_t)g, box, next_bar + 8u * (uint32_t)g);
+#pragma unroll
+            for (int k = 0; k < kLag; k++) own[k] = a.o[kGroup - kLag + k];
+#pragma unroll
+            for (int k = 0; k < kHist; k++) hist[k] = n[kGroup + k];
+        };
+#pragma unroll
+        for (int k = 0; k < kStages - 1; k++) fetch(k * kGroup);
+        Inputs even, odd;
+        take(even, 0);
+        for (int t = 0; t < s.steps; t += 2 * kGroup) {
+            fetch(t + (kStages - 1) * kGroup);
+            take(odd, t + kGroup);
+            group(even, t);
+            fetch(t + kStages * kGroup);
+            take(even, t + 2 * kGroup);
+            group(odd, t + kGroup);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+    }
+    if (dead && lane == 0) atomicExch(err, 1);
+    __syncwarp();
+    cluster_sync();  // no CTA leaves while another may still send to it
+}
+
+constexpr size_t kMaxSmem = 220 * 1024;
+size_t blur_smem(int W) { return 3 * kBandsPerCta * (size_t)blur_part(W); }
+
+}  // namespace
+
+// Maps that the cluster covers: the inboxes fit in shared memory (up to 7,500 columns) and the bands in a grid.
+bool rl_internal_blur_fits(int W, int H) {
+    return W <= (1 << 20) && blur_smem(W) <= kMaxSmem && (H - 2 + kRows - 1) / kRows <= 65535;
+}
+
+int rl_internal_blur(const rl::DevMap& m, int* err, cudaStream_t st) {
+    const int W = m.width, H = m.height;
+    Skew s;
+    s.bands = (H - 2 + kRows - 1) / kRows;
+    s.steps = blur_steps(W);
+    const size_t planes = 4 * s.plane(), edge = 3 * (size_t)s.bands * s.steps;
+    float* buf = nullptr;
+    if (int rc = rl_internal_pool_alloc((void**)&buf, (planes + edge) * sizeof(float), st)) return rc;
+    s.o = buf;
+    s.e = buf + planes;
+    cudaError_t e = cudaFuncSetAttribute(k_blur_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
+    if (e == cudaSuccess) {
+        const dim3 grid((unsigned)((s.steps + kSkewCols - 1) / kSkewCols), (unsigned)s.bands);
+        k_blur_skew<<<grid, 256, 0, st>>>(m, s);
+        k_blur_wave<<<kCtas, kThreads, blur_smem(W), st>>>(m, s, err);
+        k_blur_unskew<<<grid, 256, 0, st>>>(m, s);
+        e = cudaGetLastError();
+    }
+    cudaFreeAsync(buf, st);
+    if (e != cudaSuccess) return rl_internal_fail(RL_CUDA_ERROR, cudaGetErrorString(e));
+    return RL_OK;
+}

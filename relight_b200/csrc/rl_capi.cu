@@ -146,6 +146,7 @@ struct rl_map {
     int* d_owner = nullptr;  // rasterisation scratch: winning face per texel
     unsigned long long* d_work = nullptr;  // work-list counter of the persistent bake kernels
     char* block = nullptr;   // rl_map_create_async: every array carved from this block
+    mutable bool blurred = false;  // a blur's status word (d_work[1]) has not been read since it was queued
     ~rl_map() {
         if (block) {
             cudaFree(block);
@@ -156,6 +157,9 @@ struct rl_map {
         cudaFree(d_work);
     }
 };
+
+int rl_internal_blur(const DevMap& m, int* err, cudaStream_t st);
+bool rl_internal_blur_fits(int W, int H);
 
 // Error entry for the host-only sources of the library (e.g. the OBJ loader).
 int rl_internal_fail(int code, const char* msg) { return fail(code, "%s", msg); }
@@ -816,6 +820,17 @@ extern "C" int rl_map_add_mesh(rl_map* m, const rl_scene* s, int mesh, void* str
     return RL_OK;
 }
 
+// The status of a blur queued on `m`, read by the calls that wait for it.
+static int read_blur_status(const rl_map* m, cudaStream_t st, int* status) {
+    *status = 0;
+    if (m->blurred) CK(cudaMemcpyAsync(status, m->d_work + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    return RL_OK;
+}
+static int check_blur_status(const rl_map* m, int status) {
+    m->blurred = false;
+    return status ? fail(RL_CUDA_ERROR, "rl_map_blur: a band waited too long for the one above it") : RL_OK;
+}
+
 extern "C" int rl_map_download(const rl_map* m, int32_t* flags, int32_t* face, float* position, float* normal,
                                float* color, int32_t* photons, float* gathered, void* stream) {
     if (!m) return fail(RL_INVALID_CALL, "null map");
@@ -828,8 +843,10 @@ extern "C" int rl_map_download(const rl_map* m, int32_t* flags, int32_t* face, f
     if (color) CK(cudaMemcpyAsync(color, m->dev.color, 12 * n, cudaMemcpyDeviceToHost, st));
     if (photons) CK(cudaMemcpyAsync(photons, m->dev.photons, 4 * n, cudaMemcpyDeviceToHost, st));
     if (gathered) CK(cudaMemcpyAsync(gathered, m->dev.gathered, 12 * n, cudaMemcpyDeviceToHost, st));
+    int blur = 0;
+    if (int rc = read_blur_status(m, st, &blur)) return rc;
     CK(cudaStreamSynchronize(st));
-    return RL_OK;
+    return check_blur_status(m, blur);
 }
 
 extern "C" int rl_map_download_async(const rl_map* m, float* color, void* stream) {
@@ -2313,13 +2330,14 @@ __global__ void k_expand(DevMap m) {
     }
 }
 
-// Lightmap::blur (Lightmap.cpp:196-220).  The reference blurs in place in
-// scan order, so texel (x, y) reads the already-blurred (x-1..x+1, y-1) and
-// (x-1, y) and the original rest of its window.  Every such input has a
-// smaller t = (x-1) + 2(y-1), and texels of one t never share a window, so
-// one block walks t = 0, 1, ... with a barrier per step (a wavefront), each
-// thread owning rows y = 1 + tid, 1 + tid + blockDim, ...  Sums run in the
-// reference's window order, so the result is bit-identical.
+// Lightmap::blur (Lightmap.cpp:196-220) as one block, for the maps that the
+// cluster of rl_blur.cu does not cover (wider than its inboxes, or without
+// memory for its planes).  Texel (x, y) reads the already-blurred
+// (x-1..x+1, y-1) and (x-1, y) and the original rest of its window.  Every
+// such input has a smaller t = (x-1) + 2(y-1), and texels of one t never
+// share a window, so the block walks t = 0, 1, ... with a barrier per step,
+// each thread owning rows y = 1 + tid, 1 + tid + blockDim, ...  Sums run in
+// the reference's window order, so the result is bit-identical.
 __global__ void __launch_bounds__(1024) k_blur(DevMap m) {
     const int W = m.width, H = m.height;
     if (W < 3 || H < 3) return;
@@ -2397,6 +2415,13 @@ extern "C" int rl_map_expand(rl_map* m, void* stream) {
 
 extern "C" int rl_map_blur(rl_map* m, void* stream) {
     if (!m) return fail(RL_INVALID_CALL, "null map");
+    if (m->dev.width < 3 || m->dev.height < 3) return RL_OK;
+    if (rl_internal_blur_fits(m->dev.width, m->dev.height)) {
+        const int rc = rl_internal_blur(m->dev, reinterpret_cast<int*>(m->d_work + 1), S(stream));
+        if (rc == RL_OK) m->blurred = true;
+        if (rc != RL_OUT_OF_MEMORY) return rc;
+        cudaGetLastError();
+    }
     k_blur<<<1, 1024, 0, S(stream)>>>(m->dev);
     CK_LAUNCH("k_blur");
     return RL_OK;
@@ -2411,10 +2436,12 @@ extern "C" int rl_map_encode(const rl_map* m, int format, uint8_t* out, void* st
     if (!m || !out || format < 0 || format > 2) return fail(RL_INVALID_CALL, "rl_map_encode: bad arguments");
     cudaStream_t st = S(stream);
     long long bytes = encoded_bytes(m, format), n = (long long)m->dev.width * m->dev.height;
+    int blur = 0;
     if (format == 0) {
         CK(cudaMemcpyAsync(out, m->dev.color, bytes, cudaMemcpyDeviceToHost, st));
+        if (int rc = read_blur_status(m, st, &blur)) return rc;
         CK(cudaStreamSynchronize(st));
-        return RL_OK;
+        return check_blur_status(m, blur);
     }
     uint8_t* d = nullptr;
     if (int rc = pool_alloc((void**)&d, (size_t)bytes, st)) return rc;
@@ -2426,9 +2453,10 @@ extern "C" int rl_map_encode(const rl_map* m, int format, uint8_t* out, void* st
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(d, st);
+    if (e == cudaSuccess) rc = read_blur_status(m, st, &blur);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = fail(RL_CUDA_ERROR, "rl_map_encode: %s", cudaGetErrorString(e));
-    return rc;
+    return rc ? rc : check_blur_status(m, blur);
 }
 
 // Lightmap::save (Lightmap.cpp:223-283): RawHdr = width, height (int32)

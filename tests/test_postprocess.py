@@ -130,3 +130,24 @@ def test_gpu_blur_expand_large_maps(cuda):
             getattr(ob, op)(lm)
             assert _same(got, lm.color), (W, H, op)
             m.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(3, 3), (4, 35), (9, 34), (62, 33), (65, 66), (130, 514), (50, 549), (7600, 5)])
+def test_gpu_blur_band_edges(cuda, W, H):
+    """Blur at the edges of its bands of 32 rows (one band, one row more, the
+    first band of the second round of 16), at widths around its 8-column
+    groups and its lanes' skew, and past the widest row it hands on; two
+    blurs in a row.  Bit for bit."""
+    from relight_b200.device import DeviceMap
+    rng = np.random.default_rng(W * 1000 + H)
+    flags = (rng.random(W * H) < 0.6).astype(np.int32)
+    color = rng.uniform(-1, 4, (W * H, 3)).astype(np.float32)
+    m = DeviceMap(0, W, H)
+    m.upload(flags=flags, color=color)
+    lm = _lm(W, H, flags, color)
+    for _ in range(2):
+        m.blur()
+        ob.blur(lm)
+    assert _same(m.download(fields=("color",))["color"], lm.color)
+    m.close()
