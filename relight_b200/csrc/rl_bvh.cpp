@@ -177,11 +177,11 @@ void put_child_box4(float* dst, int slot, const Box& b) {
 }
 
 void put_child_box(float* dst, int slot, const Box& b) {
-    // n0 / n1: lo.x hi.x lo.y hi.y for child 0 / 1; n2: c0 lo.z hi.z, c1 lo.z hi.z
+    // n0 / n1: centre x y, half-extent x y of child 0 / 1; n2: centre z of both children, half-extent z of both
     float* xy = dst + 4 * slot;
-    xy[0] = b.lo[0]; xy[1] = b.hi[0]; xy[2] = b.lo[1]; xy[3] = b.hi[1];
-    dst[8 + 2 * slot] = b.lo[2];
-    dst[8 + 2 * slot + 1] = b.hi[2];
+    box_centre_half(b.lo[0], b.hi[0], &xy[0], &xy[2]);
+    box_centre_half(b.lo[1], b.hi[1], &xy[1], &xy[3]);
+    box_centre_half(b.lo[2], b.hi[2], &dst[8 + slot], &dst[10 + slot]);
 }
 
 // ---------------------------------------------------- compressed 8-wide

@@ -4,10 +4,10 @@
 //   rt::Embree::traceSegment           k_trace_segments
 //   Lightmap::initializeLumels         k_raster_owner + k_raster_init
 //   DirectLight::bakeLumel             k_direct
-//   AmbientOcclusion::bakeLumel        k_ao
+//   AmbientOcclusion::bakeLumel        k_ao, k_ao_patch (k_ao_pool: opt-in)
 //   Photons::emit/trace/store          k_photons
 //   Photonmap::gather                  k_gather
-//   IndirectLight::bakeLumel           k_indirect
+//   IndirectLight::bakeLumel           k_indirect_patch (k_indirect, k_indirect_pool: opt-in walks)
 //   RadiosityBuilder form factors      k_ff_pairs (+ host CSR assembly)
 //   hemisphere form factors            k_ff_hemi_rays + k_ff_hemi_rle + k_ff_hemi_compact
 //   radiosity gather iterations        k_jacobi4 (k_jacobi_rows per row shard)
@@ -29,6 +29,7 @@
 #include "../../include/relight_b200.h"
 #include "rl_bvh.h"
 #include "rl_device.cuh"
+#include "rl_patch.cuh"
 #include "rl_photon_records.h"
 #include "rl_lbvh.h"
 
@@ -1165,6 +1166,60 @@ __global__ void __launch_bounds__(256) k_ao(DevScene s, DevMap m, int samples, f
     col[0] = col[0] * value; col[1] = col[1] * value; col[2] = col[2] * value;
 }
 
+struct NoShade {
+    __device__ __forceinline__ V3 operator()(V3, V3, int, float, float) const { return mk3(0.f, 0.f, 0.f); }
+};
+
+__device__ __forceinline__ void ao_apply(float* col, int occluded, int samples, float fraction, float exponent) {
+    float value = 1.0f - occluded / (samples * fraction);
+    if (fabsf(1.0f - exponent) > 0.01f) value = powf(value, exponent);
+    col[0] = col[0] * value; col[1] = col[1] * value; col[2] = col[2] * value;
+}
+
+// One warp per patch of `patch` consecutive items of the iteration.
+__global__ void __launch_bounds__(256, 4) k_ao_patch(DevScene s, const __grid_constant__ DevMap m, int samples,
+                                                     float fraction, float maxd, float exponent, uint2 key,
+                                                     const __grid_constant__ Iter it, long long count, int patch,
+                                                     int refill, int* status) {
+    extern __shared__ __align__(16) char smem[];
+    PatchMem<true>& M = reinterpret_cast<PatchMem<true>*>(smem)[threadIdx.x >> 5];
+    const long long k0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * patch;
+    long long i = 0;
+    int slot = -1;
+    const int lumels = patch_load(M, m, it, k0, min(k0 + patch, count), i, slot);
+    if (lumels == 0) return;
+    patch_rays<true>(s, M, lumels, PatchRays{key, kTagAO, samples, maxd}, NoShade{}, refill, status);
+    if (slot >= 0) ao_apply(m.color + 3 * i, __float_as_int(M.acc[slot][0]), samples, fraction, exponent);
+}
+
+// How a launch over `count` iteration items is cut into patches: as many
+// lumels a warp as share a list (a list costs about 3,000 warp instructions,
+// a ray about 80) while that leaves two warps for every resident one.
+struct PatchLaunch {
+    int patch = 1;
+    unsigned grid = 0;
+    size_t smem = 0;
+    cudaError_t error = cudaSuccess;
+};
+template <bool kAny, typename K>
+static PatchLaunch patch_launch(K kernel, long long count, int samples, int threads) {
+    PatchLaunch L;
+    int dev = 0, sms = 0;
+    L.smem = sizeof(PatchMem<kAny>) * (threads / 32);
+    L.error = cudaGetDevice(&dev);
+    if (L.error == cudaSuccess) L.error = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (L.error == cudaSuccess)
+        L.error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+    L.patch = samples < (1 << 24) ? kPatch : 1;
+    while (L.patch > 1 && count < 2LL * 32 * sms * L.patch) L.patch /= 2;
+    const long long warps = (count + L.patch - 1) / L.patch;
+    L.grid = (unsigned)((warps * 32 + threads - 1) / threads);
+    return L;
+}
+// The tunable refill threshold counts lanes that wait for rays drawn on the
+// spot; here rays come ready-made, and half of it is as good.
+static int patch_refill(int lanes) { return (lanes + 1) / 2; }
+
 // AoGen over a work list of lumels (ray_loop_pool): lumel item k of the
 // iteration (items k_begin + k, k < limit), its samples in order, its colour
 // scaled when its last sample is counted — the same arithmetic as k_ao.
@@ -1262,6 +1317,20 @@ extern "C" int rl_bake_ao(const rl_scene* s, rl_map* lm, int samples, float frac
                                               g_tune[RL_TUNE_AO_REFILL], s->d_status, lm->d_work,
                                               g_tune[RL_TUNE_FG_CHUNK]);
         CK_LAUNCH("k_ao_pool");
+        return RL_OK;
+    }
+    // A patch's list costs about 3,000 warp instructions and its walk a few
+    // microseconds; up to 32 short first-hit rays a lumel are traced from the
+    // root in less (room, 256^2, 16 / 32 / 64 / 128 samples: 62 / 107 / 199 /
+    // 377 us from the root, 101 / 132 / 192 / 327 us with patches; terrain of
+    // 23k triangles, 400^2: 318 / 620 / 1,218 / 2,423 against 337 / 477 / 788 /
+    // 1,416).
+    if (samples > 32 && !wide && !wide8 && !g_tune[RL_TUNE_SPECULATIVE]) {
+        const PatchLaunch L = patch_launch<true>(k_ao_patch, count, samples, bs);
+        if (L.error != cudaSuccess) return fail(RL_CUDA_ERROR, "k_ao_patch set-up: %s", cudaGetErrorString(L.error));
+        k_ao_patch<<<L.grid, bs, L.smem, S(stream)>>>(s->dev, lm->dev, samples, fraction, maxd, exponent, key, it, count,
+                                                      L.patch, patch_refill(g_tune[RL_TUNE_AO_REFILL]), s->d_status);
+        CK_LAUNCH("k_ao_patch");
         return RL_OK;
     }
     auto kern = wide8 ? k_ao<8> : wide ? k_ao<4> : (g_tune[RL_TUNE_SPECULATIVE] ? k_ao<3> : k_ao<2>);
@@ -1569,12 +1638,61 @@ __global__ void __launch_bounds__(256, 4) k_indirect(DevScene s, DevMap m, const
     g.dir = mk3(0.f, 0.f, 0.f);
     if (kWidth == 8) ray_loop8<false>(s, g, refill, status);
     else if (kWidth == 4) ray_loop4<false>(s, g, refill, status);
-    else if (kWidth == 3) ray_loop_spec<false>(s, g, refill, status);
-    else ray_loop<false>(s, g, refill, status);
+    else ray_loop_spec<false>(s, g, refill, status);
     if (!valid) return;
     float ns = (float)samples;
     float* col = m.color + 3 * i;
     col[0] = col[0] + g.gr / ns; col[1] = col[1] + g.gg / ns; col[2] = col[2] + g.gb / ns;
+}
+
+// A final-gather sample's colour from its ray's hit, as FgGen::finish.
+struct FgShade {
+    const DevScene& s;
+    const GatherMaps& G;
+    V3 sky, amb;
+    __device__ __forceinline__ V3 operator()(V3 dir, V3 nrm, int gid, float bx, float by) const {
+        const float dp = dot3(nrm, dir);
+        const float influence = dp > 0.0f ? dp : 0.0f;
+        if (gid < 0)
+            return mk3(sky.x * influence + amb.x, sky.y * influence + amb.y, sky.z * influence + amb.z);
+        // the hit's shading record: interp3 / interp2 on the same values
+        const float4* rec = s.shade + 4 * (size_t)gid;
+        const float4 ra = __ldg(rec), rb = __ldg(rec + 1), rc = __ldg(rec + 2);
+        const V3 hn = mk3(ra.x + (rb.x - ra.x) * by + (rc.x - ra.x) * bx, ra.y + (rb.y - ra.y) * by + (rc.y - ra.y) * bx,
+                          ra.z + (rb.z - ra.z) * by + (rc.z - ra.z) * bx);
+        // a sample that adds nothing: the sums start at +0 and never turn -0, so adding 0 is the same
+        if (dot3(dir, hn) >= 0.0f) return mk3(0.f, 0.f, 0.f);
+        const float4 rv = __ldg(rec + 3);
+        const int slot = __float_as_int(rv.w);
+        if (slot < 0 || slot >= G.nmaps) return mk3(0.f, 0.f, 0.f);
+        const DevMap& P = G.maps[slot];
+        const float2 uv = make_float2(ra.w + (rb.w - ra.w) * by + (rc.w - ra.w) * bx,
+                                      rv.x + (rv.y - rv.x) * by + (rv.z - rv.x) * bx);
+        const float* g = P.gathered + 3 * (size_t)lumel_at_uv(P.width, P.height, uv);
+        return mk3(g[0] * influence + amb.x, g[1] * influence + amb.y, g[2] * influence + amb.z);
+    }
+};
+
+// One warp per patch of `patch` consecutive items of the iteration.
+__global__ void __launch_bounds__(256, 4) k_indirect_patch(DevScene s, const __grid_constant__ DevMap m,
+                                                           const __grid_constant__ GatherMaps G, int samples,
+                                                           float maxd, V3 sky, V3 amb, uint2 key,
+                                                           const __grid_constant__ Iter it, long long count, int patch,
+                                                           int refill, int* status) {
+    extern __shared__ __align__(16) char smem[];
+    PatchMem<false>& M = reinterpret_cast<PatchMem<false>*>(smem)[threadIdx.x >> 5];
+    const long long k0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * patch;
+    long long i = 0;
+    int slot = -1;
+    const int lumels = patch_load(M, m, it, k0, min(k0 + patch, count), i, slot);
+    if (lumels == 0) return;
+    patch_rays<false>(s, M, lumels, PatchRays{key, kTagFG, samples, maxd}, FgShade{s, G, sky, amb}, refill, status);
+    if (slot < 0) return;
+    const float ns = (float)samples;
+    float* col = m.color + 3 * i;
+    col[0] = col[0] + M.acc[slot][0] / ns;
+    col[1] = col[1] + M.acc[slot][1] / ns;
+    col[2] = col[2] + M.acc[slot][2] / ns;
 }
 
 // FgGen over a work list of lumels (ray_loop_pool): lumel item k of the
@@ -1676,7 +1794,15 @@ extern "C" int rl_bake_indirect(const rl_scene* s, rl_map* lm, rl_map* const* ma
         CK_LAUNCH("k_indirect_pool");
         return RL_OK;
     }
-    auto kern = wide8 ? k_indirect<8> : wide ? k_indirect<4> : (g_tune[RL_TUNE_SPECULATIVE] ? k_indirect<3> : k_indirect<2>);
+    if (!wide && !wide8 && !g_tune[RL_TUNE_SPECULATIVE]) {
+        const PatchLaunch L = patch_launch<false>(k_indirect_patch, count, samples, bs);
+        if (L.error != cudaSuccess) return fail(RL_CUDA_ERROR, "k_indirect_patch set-up: %s", cudaGetErrorString(L.error));
+        k_indirect_patch<<<L.grid, bs, L.smem, st>>>(s->dev, lm->dev, G, samples, maxd, skyv, ambv, key, it, count,
+                                                     L.patch, patch_refill(g_tune[RL_TUNE_FG_REFILL]), s->d_status);
+        CK_LAUNCH("k_indirect_patch");
+        return RL_OK;
+    }
+    auto kern = wide8 ? k_indirect<8> : wide ? k_indirect<4> : k_indirect<3>;
     kern<<<blocks_for(count, bs), bs, 0, st>>>(s->dev, lm->dev, G, samples, maxd, skyv, ambv, key, it, count,
                                               g_tune[RL_TUNE_FG_REFILL], s->d_status);
     CK_LAUNCH("k_indirect");
@@ -2536,6 +2662,8 @@ struct rl_batch {
     int slot = 0;
     long long items = 0, total[3] = {0, 0, 0};
     int grid[3] = {0, 0, 0}, block[3] = {128, 128, 128}, refill[3] = {0, 0, 0};
+    size_t smem[3] = {0, 0, 0};
+    void (*kern[3])(const BatchHeader*, unsigned long long*, int) = {nullptr, nullptr, nullptr};
     bool pool = false;  // AO / final gather through k_batch_pool (RL_TUNE_FG_POOL at creation)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -2563,89 +2691,81 @@ __device__ __forceinline__ int find_job(const long long* prefix, int njobs, long
     return lo;
 }
 
-// Persistent batch kernel for one pass kind (0 direct, 1 AO, 2 final
-// gather).  Warps take 32 work items at a time from one counter across all
-// the batch's jobs of that kind; every job's items are padded to a multiple
-// of 32, so a warp's chunk lies in one job and the scene and the ray loop's
-// warp votes are warp-uniform.  Each lane bakes one lumel with the same code
-// and Philox keys as the single-job calls, so the lumels come out
-// bit-identical to rl_bake_direct / rl_bake_ao / rl_bake_indirect.
-template <int kKind>
-__global__ void __launch_bounds__(kKind == 0 ? 128 : 256, kKind == 0 ? 1 : 4) k_batch(const BatchHeader* __restrict__ hdrs,
-                                                                  unsigned long long* counter, int refill) {
-    if (hdrs[kKind].total <= 0) return;
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        // lane 0 takes the next chunk and finds its job; the header is
-        // re-read per chunk (L1-resident) so no table state stays live in
-        // registers across the ray loop
-        unsigned long long jp = 0;
-        long long off = -1;
-        if (lane == 0) {
-            const BatchHeader* H = hdrs + kKind;
-            unsigned long long base = atomicAdd(counter + kKind, 32ull);
-            long long total = H->total;
-            if (base < (unsigned long long)total) {
-                int j = find_job(H->prefix, H->njobs, (long long)base);
-                jp = (unsigned long long)(H->jobs + j);
-                off = (long long)base - H->prefix[j];
-            }
+// The next `items` work items of kind `kind` for this warp: lane 0 takes them
+// from the counter and finds their job; every job's items are padded to a
+// multiple of 32, so they lie in one job.  Null when there are none left.
+__device__ __forceinline__ const DevJob* next_items(const BatchHeader* __restrict__ H, unsigned long long* counter,
+                                                    unsigned long long items, long long& off) {
+    // the header is re-read per chunk (L1-resident) so no table state stays
+    // live in registers across the rays
+    unsigned long long jp = 0;
+    off = -1;
+    if ((threadIdx.x & 31) == 0) {
+        const unsigned long long base = atomicAdd(counter, items);
+        if (base < (unsigned long long)H->total) {
+            const int j = find_job(H->prefix, H->njobs, (long long)base);
+            jp = (unsigned long long)(H->jobs + j);
+            off = (long long)base - H->prefix[j];
         }
-        off = __shfl_sync(0xffffffffu, off, 0);
-        if (off < 0) break;
-        jp = __shfl_sync(0xffffffffu, jp, 0);
-        const DevJob& J = *(const DevJob*)jp;
-        const long long r = off + lane;
+    }
+    off = __shfl_sync(0xffffffffu, off, 0);
+    jp = __shfl_sync(0xffffffffu, jp, 0);
+    return (const DevJob*)jp;
+}
+
+// Persistent batch kernels, one per pass kind: warps take work items from one
+// counter across all the batch's jobs of that kind.  Each lumel is baked with
+// the same code and Philox keys as the single-job calls, so it comes out
+// bit-identical to rl_bake_direct / rl_bake_ao / rl_bake_indirect.  Direct
+// light: 32 items at a time, one lumel per lane.
+__global__ void __launch_bounds__(128, 1) k_batch_direct(const BatchHeader* __restrict__ hdrs, unsigned long long* counter,
+                                                      int) {
+    long long off;
+    while (const DevJob* jp = next_items(hdrs, counter, 32, off)) {
+        const DevJob& J = *jp;
+        const long long r = off + (threadIdx.x & 31);
         long long i = 0;
-        const bool valid = r < J.count && iter_lumel(J.m, J.it, J.k_begin + r, i);
-        if (kKind == 0) {
-            if (valid) direct_lumel(J.s, J.m, *J.lights, i, J.status);
-        } else if (kKind == 1) {
-            const DevScene s = J.s;
-            AoGen g;
-            g.pos = valid ? ld3(J.m.position + 3 * i) : mk3(0.f, 0.f, 0.f);
-            g.nrm = valid ? ld3(J.m.normal + 3 * i) : mk3(0.f, 0.f, 1.f);
-            g.key = J.key;
-            g.item = (uint32_t)i;
-            g.j = 0;
-            g.stride = 1;
-            g.samples = valid ? J.samples : 0;
-            g.occluded = 0;
-            g.maxd = J.maxd;
-            __syncwarp();
-            ray_loop<true>(s, g, refill, J.status);
-            if (valid) {
-                float value = 1.0f - g.occluded / (J.samples * J.fraction);
-                if (fabsf(1.0f - J.exponent) > 0.01f) value = powf(value, J.exponent);
-                float* col = J.m.color + 3 * i;
-                col[0] = col[0] * value; col[1] = col[1] * value; col[2] = col[2] * value;
-            }
-        } else {
-            const DevScene s = J.s;
-            FgGen g;
-            g.s = &J.s;
-            g.G = J.maps;
-            g.pos = valid ? ld3(J.m.position + 3 * i) : mk3(0.f, 0.f, 0.f);
-            g.nrm = valid ? ld3(J.m.normal + 3 * i) : mk3(0.f, 0.f, 1.f);
-            g.sky = J.sky;
-            g.amb = J.amb;
-            g.key = J.key;
-            g.item = (uint32_t)i;
-            g.j = 0;
-            g.samples = valid ? J.samples : 0;
-            g.maxd = J.maxd;
-            g.gr = g.gg = g.gb = 0.f;
-            g.influence = 0.f;
-            g.dir = mk3(0.f, 0.f, 0.f);
-            __syncwarp();
-            ray_loop<false>(s, g, refill, J.status);
-            if (valid) {
-                float ns = (float)J.samples;
-                float* col = J.m.color + 3 * i;
-                col[0] = col[0] + g.gr / ns; col[1] = col[1] + g.gg / ns; col[2] = col[2] + g.gb / ns;
-            }
-        }
+        if (r < J.count && iter_lumel(J.m, J.it, J.k_begin + r, i)) direct_lumel(J.s, J.m, *J.lights, i, J.status);
         __syncwarp();
+    }
+}
+
+// AO (kKind 1) and final gather (2): a patch of kPatch items at a time, so
+// that the launch does not end on one warp's 32 lumels.
+template <int kKind>
+__global__ void __launch_bounds__(256, 4) k_batch_patch(const BatchHeader* __restrict__ hdrs,
+                                                        unsigned long long* counter, int refill) {
+    extern __shared__ __align__(16) char smem[];
+    PatchMem<kKind == 1>& M = reinterpret_cast<PatchMem<kKind == 1>*>(smem)[threadIdx.x >> 5];
+    long long off;
+    while (const DevJob* jp = next_items(hdrs + kKind, counter + kKind, kPatch, off)) {
+        const DevJob& J = *jp;
+        const DevScene s = J.s;
+        // patch_rays counts a patch's rays in 32 bits
+        const int step = J.samples < (1 << 24) ? kPatch : 1;
+        for (int q = 0; q < kPatch; q += step) {
+            long long i = 0;
+            int slot = -1;
+            const long long k0 = off + q, k1 = min(k0 + step, J.count);
+            const int lumels = patch_load(M, J.m, J.it, J.k_begin + k0, J.k_begin + k1, i, slot);
+            if (lumels == 0) continue;
+            float* col = J.m.color + 3 * i;
+            if (kKind == 1) {
+                patch_rays<kKind == 1>(s, M, lumels, PatchRays{J.key, kTagAO, J.samples, J.maxd}, NoShade{}, refill,
+                                       J.status);
+                if (slot >= 0) ao_apply(col, __float_as_int(M.acc[slot][0]), J.samples, J.fraction, J.exponent);
+            } else {
+                patch_rays<kKind == 1>(s, M, lumels, PatchRays{J.key, kTagFG, J.samples, J.maxd},
+                                       FgShade{s, *J.maps, J.sky, J.amb}, refill, J.status);
+                if (slot >= 0) {
+                    const float ns = (float)J.samples;
+                    col[0] = col[0] + M.acc[slot][0] / ns;
+                    col[1] = col[1] + M.acc[slot][1] / ns;
+                    col[2] = col[2] + M.acc[slot][2] / ns;
+                }
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -2679,7 +2799,7 @@ struct BatchSource {
 // lanes on the lumels of one job, taking the job's next chunk as lanes
 // finish instead of waiting for the chunk's slowest lumel, and moves to the
 // next job when the chunks run past its own.  Same lumels, keys and
-// arithmetic as k_batch.
+// arithmetic as k_batch_patch.
 template <int kKind>
 __global__ void __launch_bounds__(256, 4) k_batch_pool(const BatchHeader* __restrict__ hdrs,
                                                        unsigned long long* counter, int refill) {
@@ -2783,17 +2903,25 @@ static int batch_init(rl_batch* b) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     b->pool = g_tune[RL_TUNE_FG_POOL] != 0;
-    const void* kern[3] = {(const void*)k_batch<0>,
-                           b->pool ? (const void*)k_batch_pool<1> : (const void*)k_batch<1>,
-                           b->pool ? (const void*)k_batch_pool<2> : (const void*)k_batch<2>};
+    b->kern[0] = k_batch_direct;
+    b->kern[1] = b->pool ? k_batch_pool<1> : k_batch_patch<1>;
+    b->kern[2] = b->pool ? k_batch_pool<2> : k_batch_patch<2>;
     b->block[0] = 128;
     b->block[1] = g_tune[RL_TUNE_AO_BLOCK];
     b->block[2] = g_tune[RL_TUNE_FG_BLOCK];
     b->refill[1] = g_tune[RL_TUNE_AO_REFILL];
     b->refill[2] = g_tune[RL_TUNE_FG_REFILL];
+    if (!b->pool) {
+        b->smem[1] = sizeof(PatchMem<true>) * (b->block[1] / 32);
+        b->smem[2] = sizeof(PatchMem<false>) * (b->block[2] / 32);
+        for (int k = 1; k < 3; k++) {
+            b->refill[k] = patch_refill(b->refill[k]);
+            CK(cudaFuncSetAttribute(b->kern[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem[k]));
+        }
+    }
     for (int k = 0; k < 3; k++) {
         int per = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern[k], b->block[k], 0));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, b->kern[k], b->block[k], b->smem[k]));
         b->grid[k] = sms * std::max(per, 1);
     }
     return RL_OK;
@@ -3008,10 +3136,7 @@ extern "C" int rl_batch_update(rl_batch* b, const rl_batch_job* jobs, int njobs,
 static int batch_enqueue(rl_batch* b, cudaStream_t st) {
     CK(cudaMemsetAsync(b->d_counter, 0, 3 * sizeof(unsigned long long), st));
     for (int k = 0; k < 3; k++) {
-        auto kern = k == 0 ? k_batch<0>
-                    : k == 1 ? (b->pool ? k_batch_pool<1> : k_batch<1>)
-                             : (b->pool ? k_batch_pool<2> : k_batch<2>);
-        kern<<<b->grid[k], b->block[k], 0, st>>>(b->d_hdr, b->d_counter, b->refill[k]);
+        b->kern[k]<<<b->grid[k], b->block[k], b->smem[k], st>>>(b->d_hdr, b->d_counter, b->refill[k]);
         CK_LAUNCH("k_batch");
     }
     return RL_OK;

@@ -18,10 +18,11 @@ namespace rl {
 // ------------------------------------------------------------------ scene
 
 // BVH node, 64 bytes, both children's boxes in the parent (four float4):
-//   n0 = c0.lo.x c0.hi.x c0.lo.y c0.hi.y
-//   n1 = c1.lo.x c1.hi.x c1.lo.y c1.hi.y
-//   n2 = c0.lo.z c0.hi.z c1.lo.z c1.hi.z
+//   n0 = child 0's centre x y, half-extent x y
+//   n1 = child 1's centre x y, half-extent x y
+//   n2 = centre z of child 0 and 1, half-extent z of child 0 and 1
 //   n3 = child0, child1 (int bits), 0, 0
+// (box_centre_half: the pairs that the packed slab test takes lie side by side)
 // child >= 0: inner node index; child < 0: leaf, ~child = first_tri << 3 | (count - 1).
 // Triangles, 48 bytes in leaf order: t0 = v0.xyz | gid bits, t1 = e1.xyz, t2 = e2.xyz.
 struct DevScene {
@@ -266,21 +267,69 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     return r;
 }
 
+// Packed single precision: two multiply-adds in one instruction.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// 1 / d for the slab test only: one unit in the last place is far inside the
+// boxes' padding.  |d| below 1e-20 is taken as +-1e-20, to keep it finite.
+__device__ __forceinline__ float slab_inv(float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d) < 1e-20f ? copysignf(1e-20f, d) : d));
+    return r;
+}
+
+// What the slab test of a ray needs: 1 / d, -o / d, |1 / d| and -|1 / d|, x
+// and y packed, z twice (the z of a node's two children is one operand).
+struct Slab {
+    f32x2 ixy, oxy, axy, bxy, iz, oz, az, bz;
+};
+__device__ __forceinline__ Slab make_slab(V3 o, V3 d) {
+    const float ix = slab_inv(d.x), iy = slab_inv(d.y), iz = slab_inv(d.z);
+    const float ax = fabsf(ix), ay = fabsf(iy), az = fabsf(iz);
+    const float oz = -(o.z * iz);
+    Slab s;
+    s.ixy = pack2(ix, iy);
+    s.oxy = pack2(-(o.x * ix), -(o.y * iy));
+    s.axy = pack2(ax, ay);
+    s.bxy = pack2(-ax, -ay);
+    s.iz = pack2(iz, iz);
+    s.oz = pack2(oz, oz);
+    s.az = pack2(az, az);
+    s.bz = pack2(-az, -az);
+    return s;
+}
+
 // Slab test of both children of a node against [tnear, tmax]; returns the
 // entry distances.  Conservative: boxes were padded at build and the exit
-// bound is widened by a few ulps.
-__device__ __forceinline__ void slab2(float4 n0, float4 n1, float4 n2, V3 idir, V3 ood, float tnear, float tmax,
-                                      bool& h0, bool& h1, float& e0, float& e1) {
-    float a0 = __fmaf_rn(n0.x, idir.x, -ood.x), a1 = __fmaf_rn(n0.y, idir.x, -ood.x);
-    float b0 = __fmaf_rn(n0.z, idir.y, -ood.y), b1 = __fmaf_rn(n0.w, idir.y, -ood.y);
-    float c0 = __fmaf_rn(n2.x, idir.z, -ood.z), c1 = __fmaf_rn(n2.y, idir.z, -ood.z);
-    float lo0 = fmax3(fminf(a0, a1), fminf(b0, b1), fmaxf(fminf(c0, c1), tnear));
-    float hi0 = fmin3(fmaxf(a0, a1), fmaxf(b0, b1), fminf(fmaxf(c0, c1), tmax));
-    float d0 = __fmaf_rn(n1.x, idir.x, -ood.x), d1 = __fmaf_rn(n1.y, idir.x, -ood.x);
-    float f0 = __fmaf_rn(n1.z, idir.y, -ood.y), f1 = __fmaf_rn(n1.w, idir.y, -ood.y);
-    float g0 = __fmaf_rn(n2.z, idir.z, -ood.z), g1 = __fmaf_rn(n2.w, idir.z, -ood.z);
-    float lo1 = fmax3(fminf(d0, d1), fminf(f0, f1), fmaxf(fminf(g0, g1), tnear));
-    float hi1 = fmin3(fmaxf(d0, d1), fmaxf(f0, f1), fminf(fmaxf(g0, g1), tmax));
+// bound is widened by a few ulps.  With boxes as centre and half-extent, entry
+// and exit are (c - o) / d -+ h / |d|: no minimum and maximum per axis, and
+// nine packed multiply-adds for both boxes (against twelve and twelve more
+// minima and maxima with the planes; terrain final gather 25.8 -> 25.1 ms).
+__device__ __forceinline__ void slab2(float4 n0, float4 n1, float4 n2, const Slab& r, float tnear, float tmax, bool& h0,
+                                      bool& h1, float& e0, float& e1) {
+    const f32x2 t0 = fma2(pack2(n0.x, n0.y), r.ixy, r.oxy), t1 = fma2(pack2(n1.x, n1.y), r.ixy, r.oxy);
+    const f32x2 tz = fma2(pack2(n2.x, n2.y), r.iz, r.oz);
+    const f32x2 w0 = pack2(n0.z, n0.w), w1 = pack2(n1.z, n1.w), wz = pack2(n2.z, n2.w);
+    const float2 a0 = unpack2(fma2(w0, r.bxy, t0)), b0 = unpack2(fma2(w0, r.axy, t0));
+    const float2 a1 = unpack2(fma2(w1, r.bxy, t1)), b1 = unpack2(fma2(w1, r.axy, t1));
+    const float2 az = unpack2(fma2(wz, r.bz, tz)), bz = unpack2(fma2(wz, r.az, tz));
+    const float lo0 = fmax3(a0.x, a0.y, fmaxf(az.x, tnear)), hi0 = fmin3(b0.x, b0.y, fminf(bz.x, tmax));
+    const float lo1 = fmax3(a1.x, a1.y, fmaxf(az.y, tnear)), hi1 = fmin3(b1.x, b1.y, fminf(bz.y, tmax));
     h0 = lo0 <= hi0 * 1.0000003f;
     h1 = lo1 <= hi1 * 1.0000003f;
     e0 = lo0;
@@ -295,8 +344,7 @@ __device__ __forceinline__ bool traverse(const DevScene& s, V3 o, V3 d, float tn
                                          int* overflow) {
     hit.gid = -1;
     if (s.ntris == 0) return false;
-    V3 idir = mk3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-    V3 ood = mk3(o.x * idir.x, o.y * idir.y, o.z * idir.z);
+    const Slab slab = make_slab(o, d);
     int stack[kStackSize];
     int sp = 0;
     int node = 0;
@@ -308,7 +356,7 @@ __device__ __forceinline__ bool traverse(const DevScene& s, V3 o, V3 d, float tn
             float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
             bool h0, h1;
             float e0, e1;
-            slab2(n0, n1, n2, idir, ood, tnear, best, h0, h1, e0, e1);
+            slab2(n0, n1, n2, slab, tnear, best, h0, h1, e0, e1);
             int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
             if (h0 && h1) {
                 int nearc = c0, farc = c1;
@@ -350,16 +398,15 @@ __device__ __forceinline__ bool traverse(const DevScene& s, V3 o, V3 d, float tn
 
 constexpr int kNodeDone = (int)0x80000000;  // never a leaf code: ntris < 2^28
 
-// Persistent per-lane ray loop.  A generator `g` supplies this lane's rays
-// one after another (g.next) and consumes each result (g.finish).  A lane
-// starts its next ray as soon as its current one terminates, so lanes of a
-// warp never wait for each other between rays — only inside one traversal
-// step (the inner-node loop, then one leaf).  Results are the same as
-// traverse<kAny>() per ray: closest hit with the smaller-id tie-break, or
-// first hit.
+// Per-lane ray loop.  A generator `g` supplies this lane's rays one after
+// another (g.next) and consumes each result (g.finish).  Lanes whose ray ended
+// wait until `refill` of the warp's live lanes have ended, then start their
+// next rays together, so ray generation and hit shading run on many lanes at
+// once.  Results are those of traverse<kAny>() per ray.
 template <bool kAny, typename Gen>
 __device__ __forceinline__ void ray_loop(const DevScene& s, Gen& g, int refill, int* overflow) {
-    V3 o = mk3(0.f, 0.f, 0.f), d = o, idir = o, ood = o;
+    V3 o = mk3(0.f, 0.f, 0.f), d = o;
+    Slab slab = make_slab(o, d);
     float tnear = 0.f, tfar = 0.f, best = 0.f;
     int best_gid = 0x7fffffff;
     RayHit hit;
@@ -384,8 +431,7 @@ __device__ __forceinline__ void ray_loop(const DevScene& s, Gen& g, int refill, 
             }
             if (g.next(o, d, tnear, tfar)) {
                 have = true;
-                idir = mk3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-                ood = mk3(o.x * idir.x, o.y * idir.y, o.z * idir.z);
+                slab = make_slab(o, d);
                 best = tfar;
                 best_gid = 0x7fffffff;
                 hit.gid = -1;
@@ -402,7 +448,7 @@ __device__ __forceinline__ void ray_loop(const DevScene& s, Gen& g, int refill, 
             float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
             bool h0, h1;
             float e0, e1;
-            slab2(n0, n1, n2, idir, ood, tnear, best, h0, h1, e0, e1);
+            slab2(n0, n1, n2, slab, tnear, best, h0, h1, e0, e1);
             int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
             if (h0 && h1) {
                 int nearc = c0, farc = c1;
@@ -440,15 +486,13 @@ __device__ __forceinline__ void ray_loop(const DevScene& s, Gen& g, int refill, 
     }
 }
 
-// ray_loop over a shared list of work items (lumels) instead of one per
-// lane: a lane whose item has no rays left takes the next item from its
-// warp's pool, and the warp refills the pool from `src` (src.claim(lo, hi):
-// called by the whole warp, gives the same [lo, hi) to every lane, false
-// when the source is dry).  Lanes therefore keep tracing until the source
-// runs dry, instead of idling until the warp's slowest item is done, and a
-// persistent grid has no wave tail.  Neighbouring items of a chunk stay in
-// one warp (coherent rays).  Each item is still one lane's rays in order,
-// so results are those of ray_loop.  The generator adds:
+// ray_loop over a shared list of work items (lumels) instead of one per lane
+// (opt-in, RL_TUNE_FG_POOL): a lane whose item has no rays left takes the next
+// item from its warp's pool, and the warp refills the pool from `src`
+// (src.claim(lo, hi): called by the whole warp, gives the same [lo, hi) to
+// every lane, false when the source is dry).  Neighbouring items of a chunk
+// stay in one warp (coherent rays).  Each item is still one lane's rays in
+// order, so results are those of ray_loop.  The generator adds:
 //   has_more()        the current item has rays left
 //   end_item()        the current item is done (write its result); no-op
 //                     when the lane holds none
@@ -473,7 +517,8 @@ struct CounterSource {
 
 template <bool kAny, typename Gen, typename Src>
 __device__ __forceinline__ void ray_loop_pool(const DevScene& s, Gen& g, int refill, int* overflow, Src& src) {
-    V3 o = mk3(0.f, 0.f, 0.f), d = o, idir = o, ood = o;
+    V3 o = mk3(0.f, 0.f, 0.f), d = o;
+    Slab slab = make_slab(o, d);
     float tnear = 0.f, tfar = 0.f, best = 0.f;
     int best_gid = 0x7fffffff;
     RayHit hit;
@@ -516,8 +561,7 @@ __device__ __forceinline__ void ray_loop_pool(const DevScene& s, Gen& g, int ref
             if (need && !exhausted) {
                 g.next(o, d, tnear, tfar);
                 have = true;
-                idir = mk3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-                ood = mk3(o.x * idir.x, o.y * idir.y, o.z * idir.z);
+                slab = make_slab(o, d);
                 best = tfar;
                 best_gid = 0x7fffffff;
                 hit.gid = -1;
@@ -532,7 +576,7 @@ __device__ __forceinline__ void ray_loop_pool(const DevScene& s, Gen& g, int ref
             float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
             bool h0, h1;
             float e0, e1;
-            slab2(n0, n1, n2, idir, ood, tnear, best, h0, h1, e0, e1);
+            slab2(n0, n1, n2, slab, tnear, best, h0, h1, e0, e1);
             int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
             if (h0 && h1) {
                 int nearc = c0, farc = c1;
@@ -570,9 +614,12 @@ __device__ __forceinline__ void ray_loop_pool(const DevScene& s, Gen& g, int ref
     }
 }
 
+// Opt-in ray loops over the lanes' own lumels (RL_TUNE_SPECULATIVE,
+// RL_TUNE_BVH_WIDTH), with ray_loop's refill rule.
 template <bool kAny, typename Gen>
 __device__ __forceinline__ void ray_loop_spec(const DevScene& s, Gen& g, int refill, int* overflow) {
-    V3 o = mk3(0.f, 0.f, 0.f), d = o, idir = o, ood = o;
+    V3 o = mk3(0.f, 0.f, 0.f), d = o;
+    Slab slab = make_slab(o, d);
     float tnear = 0.f, tfar = 0.f, best = 0.f;
     int best_gid = 0x7fffffff;
     RayHit hit;
@@ -597,8 +644,7 @@ __device__ __forceinline__ void ray_loop_spec(const DevScene& s, Gen& g, int ref
             }
             if (g.next(o, d, tnear, tfar)) {
                 have = true;
-                idir = mk3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-                ood = mk3(o.x * idir.x, o.y * idir.y, o.z * idir.z);
+                slab = make_slab(o, d);
                 best = tfar;
                 best_gid = 0x7fffffff;
                 hit.gid = -1;
@@ -619,7 +665,7 @@ __device__ __forceinline__ void ray_loop_spec(const DevScene& s, Gen& g, int ref
             float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
             bool h0, h1;
             float e0, e1;
-            slab2(n0, n1, n2, idir, ood, tnear, best, h0, h1, e0, e1);
+            slab2(n0, n1, n2, slab, tnear, best, h0, h1, e0, e1);
             int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
             if (h0 && h1) {
                 int nearc = c0, farc = c1;
@@ -898,15 +944,15 @@ __device__ __forceinline__ void visit8(const DevScene& s, int node, V3 idir, V3 
     tmask = t;
 }
 
-// ray_loop over the compressed 8-wide tree: node groups (a node's internal
+// The ray loop over the compressed 8-wide tree: node groups (a node's internal
 // children hit, as key bits, with its child base) on the stack instead of
 // single nodes, and the triangles of the leaf children hit tested in the
 // following step (Ylitie, Karras & Laine, "Efficient incoherent ray traversal
 // on GPUs through compressed wide BVHs", HPG 2017).  Same warp refill and
-// same closest-hit / tie-break rule as ray_loop, so the hits are identical.
+// same closest-hit / tie-break rule, so the hits are identical.
 // On the terrain final gather it measured 2.3x slower than the binary walk
 // (116 vs 51 ms): each visit decodes and tests eight boxes and the octant
-// order culls less than ray_loop's distance order, so it is opt-in.
+// order culls less than a distance order, so it is opt-in.
 template <bool kAny, typename Gen>
 __device__ __forceinline__ void ray_loop8(const DevScene& s, Gen& g, int refill, int* overflow) {
     V3 o = mk3(0.f, 0.f, 0.f), d = o, idir = o, ood = o;

@@ -17,6 +17,7 @@
 
 #include <cstdint>
 
+#include "rl_bvh.h"
 #include "rl_lbvh.h"
 
 namespace rl {
@@ -128,6 +129,16 @@ __device__ __forceinline__ void load_box(const float* nbox, const float* tbox, c
     }
 }
 
+// Both children's boxes (lo xyz, hi xyz) in the traversal layout.
+__device__ __forceinline__ void put_boxes(float* dst, const float a[6], const float b[6]) {
+    box_centre_half(a[0], a[3], dst + 0, dst + 2);
+    box_centre_half(a[1], a[4], dst + 1, dst + 3);
+    box_centre_half(b[0], b[3], dst + 4, dst + 6);
+    box_centre_half(b[1], b[4], dst + 5, dst + 7);
+    box_centre_half(a[2], a[5], dst + 8, dst + 10);
+    box_centre_half(b[2], b[5], dst + 9, dst + 11);
+}
+
 // Bottom-up pass, one thread per leaf: the second thread to reach an internal
 // node writes the node (both children's boxes) and its union box, then climbs.
 __global__ void k_lbvh_up(const unsigned long long* keys, int n, const int* child, const int* parent_int,
@@ -144,9 +155,7 @@ __global__ void k_lbvh_up(const unsigned long long* keys, int n, const int* chil
         load_box(nbox, tbox, keys, c0, a);
         load_box(nbox, tbox, keys, c1, b);
         float* dst = nodes + 16 * (size_t)p;
-        dst[0] = a[0]; dst[1] = a[3]; dst[2] = a[1]; dst[3] = a[4];
-        dst[4] = b[0]; dst[5] = b[3]; dst[6] = b[1]; dst[7] = b[4];
-        dst[8] = a[2]; dst[9] = a[5]; dst[10] = b[2]; dst[11] = b[5];
+        put_boxes(dst, a, b);
         int code0 = c0 >= 0 ? c0 : ~(((~c0) << 3) | 0);
         int code1 = c1 >= 0 ? c1 : ~(((~c1) << 3) | 0);
         dst[12] = __int_as_float(code0);
@@ -184,8 +193,7 @@ __global__ void k_lbvh_tris(const unsigned long long* keys, int n, const float* 
 __global__ void k_lbvh_single(const float* tbox, float* nodes) {
     float a[6];
     for (int k = 0; k < 6; k++) a[k] = tbox[k];
-    float vals[12] = {a[0], a[3], a[1], a[4], a[0], a[3], a[1], a[4], a[2], a[5], a[2], a[5]};
-    for (int k = 0; k < 12; k++) nodes[k] = vals[k];
+    put_boxes(nodes, a, a);
     int code = ~0;
     nodes[12] = __int_as_float(code);
     nodes[13] = __int_as_float(code);
