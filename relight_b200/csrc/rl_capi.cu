@@ -3,7 +3,7 @@
 // Kernel map (reference function -> kernel):
 //   rt::Embree::traceSegment           k_trace_segments
 //   Lightmap::initializeLumels         k_raster_owner + k_raster_init
-//   DirectLight::bakeLumel             k_direct
+//   DirectLight::bakeLumel             k_direct, k_direct_group
 //   AmbientOcclusion::bakeLumel        k_ao, k_ao_patch (k_ao_pool: opt-in)
 //   Photons::emit/trace/store          k_photons
 //   Photonmap::gather                  k_gather
@@ -1043,6 +1043,85 @@ __global__ void k_direct(DevScene s, DevMap m, const __grid_constant__ LightTabl
     direct_lumel(s, m, T, i, status);
 }
 
+// `group` lanes (a power of two) per lumel, for maps too small to fill the GPU
+// with one: the lanes trace the lumel's light samples between them, `group` at
+// a time, and then every lane of the group adds their influences in the order
+// of direct_lumel's loops, with its arithmetic.  A lane's sample is the q-th
+// of all the lights'; the lights are copied to shared memory, where lanes may
+// look at different ones.
+__global__ void __launch_bounds__(128) k_direct_group(DevScene s, const __grid_constant__ DevMap m,
+                                                      const __grid_constant__ LightTable T,
+                                                      const __grid_constant__ Iter it, long long count, int group,
+                                                      int* status) {
+    extern __shared__ __align__(16) char smem[];
+    rl_light* lights = reinterpret_cast<rl_light*>(smem);
+    float* verts = reinterpret_cast<float*>(lights + T.n);
+    for (int w = threadIdx.x; w < T.n * (int)(sizeof(rl_light) / 4); w += blockDim.x)
+        reinterpret_cast<int*>(lights)[w] = reinterpret_cast<const int*>(T.l)[w];
+    for (int w = threadIdx.x; w < 3 * T.nverts; w += blockDim.x) verts[w] = T.verts[w];
+    __syncthreads();
+    const int part = threadIdx.x & (group - 1);
+    const long long k = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / group;
+    long long i = 0;
+    const bool valid = k < count && iter_lumel(m, it, k, i);
+    V3 pos = mk3(0.f, 0.f, 0.f), nrm = pos;
+    float cr = 0.f, cg = 0.f, cb = 0.f;
+    float* col = m.color + 3 * i;
+    if (valid) {
+        pos = ld3(m.position + 3 * i);
+        nrm = ld3(m.normal + 3 * i);
+        cr = col[0]; cg = col[1]; cb = col[2];
+    }
+    const unsigned members = __ballot_sync(0xffffffffu, valid);  // whole groups
+    if (!valid) return;
+    V3 acc = mk3(0.f, 0.f, 0.f);
+    int l = 0, v = 0;    // the sample that is added next
+    int ql = 0, qv = 0;  // this lane's sample, `part` further on
+    auto samples = [&](int light) { return lights[light].vertex_count > 0 ? lights[light].vertex_count : 1; };
+    auto advance = [&](int& light, int& at, int by) {
+        at += by;
+        while (light < T.n && at >= samples(light)) {
+            at -= samples(light);
+            light++;
+        }
+    };
+    advance(ql, qv, part);
+    while (l < T.n) {
+        float inf = 0.f;
+        if (ql < T.n) {
+            const rl_light& L = lights[ql];
+            V3 p = ld3(L.position);
+            if (L.vertex_count > 0) p = add3(ld3(verts + 3 * (L.vertex_first + qv)), p);
+            inf = influence_from_point(s, pos, nrm, p, L, status);
+        }
+        __syncwarp(members);
+        for (int j = 0; j < group && l < T.n; j++) {
+            const float f = __shfl_sync(members, inf, j, group);
+            const rl_light& L = lights[l];
+            const V3 add = mul3(mul3(ld3(L.color), L.intensity), f);
+            if (L.vertex_count > 0) {
+                if (f > 0.0f) acc = add3(acc, add);
+                if (++v == L.vertex_count) {
+                    const float n = (float)L.vertex_count;
+                    cr = cr + acc.x / n; cg = cg + acc.y / n; cb = cb + acc.z / n;
+                    acc = mk3(0.f, 0.f, 0.f);
+                    v = 0;
+                    l++;
+                }
+            } else {
+                // direct_lumel adds a zero where there is no influence
+                cr = cr + (f > 0.0f ? add.x : 0.f); cg = cg + (f > 0.0f ? add.y : 0.f);
+                cb = cb + (f > 0.0f ? add.z : 0.f);
+                l++;
+            }
+        }
+        advance(ql, qv, group);
+    }
+    if (part == 0) {
+        col[0] = cr; col[1] = cg; col[2] = cb;
+    }
+}
+
 // Validate an rl_iterator (NULL = LumelBakeIterator(0, 1)) and size the
 // launch: one thread per visited lumel (kind 0) or per lumel (kind 1).
 static int make_iter(const rl_iterator* it, const rl_scene* s, long long n, Iter& out, long long& count) {
@@ -1084,6 +1163,27 @@ extern "C" int rl_bake_direct(const rl_scene* s, rl_map* lm, const rl_light* lig
     if (rc) return rc;
     if (count == 0 || nlights == 0) return RL_OK;
     tile_whole_map(it, count, lm->dev);
+    long long rays = 0;
+    for (int l = 0; l < nlights; l++) rays += std::max(lights[l].vertex_count, 1);
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // Lanes per lumel: up to about one thread for every resident one (lumels
+    // that trace alone leave small maps to 18 rays in series: room, 48^2 / 100^2
+    // / 256^2: 87 / 91 / 90 us with one lane, 38 / 40 / 66 us with 16, 16 and
+    // 4); four times as many where alpha tests make the shadow rays long and
+    // uneven (textured room, 48^2 / 256^2 / 384^2: 261 / 557 / 504 us with one
+    // lane, 53 / 100 / 120 us with 16, 16 and 8).
+    const long long most = (s->dev.has_alpha ? 8192LL : 2048LL) * sms;
+    int group = 1;
+    while (group < 16 && group < rays && count * group * 2 <= most) group *= 2;
+    if (group > 1) {
+        const size_t smem = sizeof(rl_light) * (size_t)T.n + 12 * (size_t)T.nverts;
+        k_direct_group<<<blocks_for(count * group, 128), 128, smem, S(stream)>>>(s->dev, lm->dev, T, it, count, group,
+                                                                                 s->d_status);
+        CK_LAUNCH("k_direct_group");
+        return RL_OK;
+    }
     k_direct<<<blocks_for(count, 128), 128, 0, S(stream)>>>(s->dev, lm->dev, T, it, count, s->d_status);
     CK_LAUNCH("k_direct");
     return RL_OK;
