@@ -1,10 +1,10 @@
 """Kernels that split a map's work by its size, against the oracle, bit for
-bit: direct light with several lanes per lumel."""
+bit: direct light with several lanes per lumel and the staged photon gather."""
 import numpy as np
 import pytest
 
-from oracle_bind import Oracle
-from relight_b200 import scenes
+from oracle_bind import LumelMap, Oracle
+from relight_b200 import _abi, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +29,22 @@ def test_direct_light_lane_groups(cuda, size, textured):
         assert lm.color.any() or size == 24
         assert np.array_equal(got.view(np.uint32), lm.color.view(np.uint32)), spec
     assert ds.status() == 0
+
+
+@pytest.mark.parametrize("W,H,radius", [(64, 64, 7), (65, 63, 7), (130, 70, 0), (70, 66, 3), (40, 33, 15), (40, 33, 16)])
+def test_photon_gather_tiles(cuda, W, H, radius):
+    """Edges of the 64 x 8 tiles and of the radii that are staged, with
+    negative colours and texels without photons."""
+    from relight_b200.device import DeviceMap
+    rng = np.random.default_rng(W * 100 + H + radius)
+    n = W * H
+    pm = LumelMap(W, H)
+    pm.color[:] = rng.uniform(-1, 2, (n, 3))
+    pm.photons[:] = rng.integers(0, 3, n) * (rng.random(n) < 0.3)
+    m = DeviceMap(1, W, H)
+    m.upload(color=pm.color, photons=pm.photons)
+    _abi.check(_abi.lib().rl_photonmap_gather(m.handle, radius, None))
+    got = m.download(fields=("gathered",))["gathered"]
+    Oracle(scenes.room_scene(size=16).scene.flat).gather(pm, radius)
+    assert np.array_equal(got.view(np.uint32), pm.gathered.view(np.uint32))
+    m.close()
