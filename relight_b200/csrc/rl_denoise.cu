@@ -1160,45 +1160,127 @@ __global__ void k_dn_up_bwd(const bf16* gout, bf16* gin, int C, int W, int H, in
     }
 }
 
-// db[c] += sum over pixels of g[p][c], c < cout (blockDim.x = channel stride).
-__global__ void k_dn_bias_grad(const bf16* g, int cs, int cout, long long P, float* db) {
-    const int c = threadIdx.x;
-    float s = 0.f;
-    for (long long p = blockIdx.x; p < P; p += gridDim.x) s += bf(g[p * cs + c]);
-    if (c < cout) atomicAdd(db + c, s);
+// One layer's piece of the bias-gradient and optimiser launches, which take
+// all eight layers in one go: a launch per layer and tensor (8 + 16 + 8 of
+// 3 to 10 us each, most of it latency) took 170 us of a training step's 800.
+struct LayerGrad {
+    const bf16* g;  // gradient activations [pixels][cs]
+    int cs, cout;
+    long long pixels;
+    float* db;
+    int block0;     // first block of this layer
+};
+struct LayerGrads {
+    LayerGrad l[8];
+};
+constexpr int kBiasThreads = 256, kBiasPixels = 2048;  // pixels per block
+
+// db[c] += sum over pixels of g[p][c], c < cout.  A thread sums 8 channels
+// (16 bytes) of every (256 / (cs / 8))-th pixel of its block's share; cs / 8
+// divides 256 or is at most 16 (idle threads at the end otherwise).
+__global__ void __launch_bounds__(kBiasThreads) k_dn_bias_grad(const __grid_constant__ LayerGrads L) {
+    __shared__ float sum[kBiasThreads][8];
+    int li = 0;
+    while (li < 7 && (int)blockIdx.x >= L.l[li + 1].block0) li++;
+    const LayerGrad& G = L.l[li];
+    const int groups = G.cs / 8, lanes = kBiasThreads / groups;  // pixels side by side
+    const int grp = threadIdx.x % groups, px = threadIdx.x / groups;
+    const long long p0 = (long long)(blockIdx.x - G.block0) * kBiasPixels;
+    const long long p1 = p0 + kBiasPixels < G.pixels ? p0 + kBiasPixels : G.pixels;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (px < lanes)
+#pragma unroll 4
+        for (long long p = p0 + px; p < p1; p += lanes) {
+            Pack8 v;
+            v.u = reinterpret_cast<const uint4*>(G.g + p * G.cs)[grp];
+#pragma unroll
+            for (int k = 0; k < 8; k++) s[k] += bf(v.h[k]);
+        }
+#pragma unroll
+    for (int k = 0; k < 8; k++) sum[threadIdx.x][k] = s[k];
+    __syncthreads();
+    for (int c = threadIdx.x; c < G.cout; c += kBiasThreads) {
+        float t = 0.f;
+        for (int q = 0; q < lanes; q++) t += sum[q * groups + c / 8][c % 8];
+        atomicAdd(G.db + c, t);
+    }
 }
 
 // L1 loss on log1p colours: pred = y[:3] + x[:3]; gy = sign(pred - t) * valid * scale.
-__global__ void k_dn_loss(const bf16* y, const bf16* x, const float4* t, long long P, float scale, bf16* gy,
-                          float* loss) {
+__global__ void __launch_bounds__(256) k_dn_loss(const bf16* y, const bf16* x, const float4* t, long long P, float scale,
+                                                 bf16* gy, float* loss) {
+    __shared__ float warp_sum[8];
     float acc = 0.f;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
-        float4 tt = t[p];
-        float tv[3] = {tt.x, tt.y, tt.z};
-        for (int c = 0; c < kFeat; c++) {
-            float g = 0.f;
-            if (c < 3 && tt.w > 0.f) {
-                float d = bf(y[p * kFeat + c]) + bf(x[p * kFeat + c]) - tv[c];
+        const float4 tt = t[p];
+        const float tv[3] = {tt.x, tt.y, tt.z};
+        Pack8 yv, xv, g;
+        yv.u = reinterpret_cast<const uint4*>(y + p * kFeat)[0];
+        xv.u = reinterpret_cast<const uint4*>(x + p * kFeat)[0];
+        g.u = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            if (tt.w > 0.f) {
+                const float d = bf(yv.h[c]) + bf(xv.h[c]) - tv[c];
                 acc += fabsf(d);
-                g = (d > 0.f ? 1.f : d < 0.f ? -1.f : 0.f) * scale;
+                g.h[c] = __float2bfloat16((d > 0.f ? 1.f : d < 0.f ? -1.f : 0.f) * scale);
             }
-            gy[p * kFeat + c] = __float2bfloat16(g);
-        }
+        uint4* o = reinterpret_cast<uint4*>(gy + p * kFeat);
+        o[0] = g.u;
+        o[1] = make_uint4(0u, 0u, 0u, 0u);
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, acc * scale);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0 && loss) {
+        for (int w = 1; w < 8; w++) acc += warp_sum[w];
+        atomicAdd(loss, acc * scale);
+    }
 }
 
-__global__ void k_dn_adam(float* p, float* g, float* m, float* v, long long n, float lr, float b1, float b2, float eps,
-                          float bc1, float bc2) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float gi = g[i];
-        float mi = b1 * m[i] + (1.f - b1) * gi;
-        float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-        g[i] = 0.f;
+// Adam on one layer's tensors, and the layer's packed operands with it.
+struct LayerStep {
+    float *w, *gw, *mw, *vw, *b, *gb, *mb, *vb, *bias;
+    bf16 *wp, *wt;
+    int cout, ncols, seg0, seg1, kpad;
+    int block0;  // first block of this layer (kAdamThreads weights each; the last one takes the biases)
+};
+struct LayerSteps {
+    LayerStep l[8];
+};
+constexpr int kAdamThreads = 256;
+
+__device__ __forceinline__ float adam(float* p, float* g, float* m, float* v, long long i, float lr, float b1, float b2,
+                                      float eps, float bc1, float bc2) {
+    const float gi = g[i];
+    const float mi = b1 * m[i] + (1.f - b1) * gi;
+    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float r = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    p[i] = r;
+    g[i] = 0.f;
+    return r;
+}
+
+// One step of every layer.  Each weight goes straight to its place in both
+// packed operands (k_dn_pack's layouts, whose padding stays zero from there).
+__global__ void __launch_bounds__(kAdamThreads) k_dn_adam(const __grid_constant__ LayerSteps L, float lr, float b1,
+                                                          float b2, float eps, float bc1, float bc2) {
+    int li = 0;
+    while (li < 7 && (int)blockIdx.x >= L.l[li + 1].block0) li++;
+    const LayerStep& S = L.l[li];
+    const int row = 9 * S.kpad, n = S.cout * row;
+    const int i = (int)(blockIdx.x - S.block0) * kAdamThreads + threadIdx.x;
+    if (i < n) {
+        const bf16 w = __float2bfloat16(adam(S.w, S.gw, S.mw, S.vw, i, lr, b1, b2, eps, bc1, bc2));
+        const int co = i / row, q = i - co * row, tap = q / S.kpad, col = q - tap * S.kpad;
+        const int k0 = (S.seg0 + 15) / 16 * 16, K = k0 + (S.seg1 + 15) / 16 * 16, s1 = (S.seg0 + 63) / 64 * 64;
+        const int kk = col < S.seg0 ? col : col >= s1 && col - s1 < S.seg1 ? k0 + col - s1 : -1;
+        if (kk >= 0) S.wp[(((size_t)tap * (K / 8) + kk / 8) * S.ncols + co) * 8 + kk % 8] = w;
+        S.wt[(((size_t)(8 - tap) * (S.ncols / 8) + co / 8) * S.kpad + col) * 8 + co % 8] = w;
+    } else if (i - n < S.cout) {
+        S.bias[i - n] = adam(S.b, S.gb, S.mb, S.vb, i - n, lr, b1, b2, eps, bc1, bc2);
     }
 }
 
@@ -1437,12 +1519,12 @@ int conv_wgrad(rl_denoiser* d, int l, const bf16* gout, const bf16* in0, const b
         if (int rc = rl_dn_conv3x3_wgrad(gout, c.cout, c.ncols, in1, c.segs[1], c.segs[1], w, h, n, c.gw,
                                          pad64(c.segs[0]), c.kpad, d->d_err, st))
             return rc;
-    const long long P = (long long)n * w * h;
-    k_dn_bias_grad<<<(int)std::min<long long>(P, 2048), c.ncols, 0, st>>>(gout, c.ncols, c.cout, P, c.gb);
     return RL_OK;
 }
 
-int forward(rl_denoiser* d, int n, int h, int w, cudaStream_t st) {
+// x and y: the network's input and output, the denoiser's own buffers or the
+// caller's (16-byte aligned).
+int forward(rl_denoiser* d, const bf16* x, bf16* y, int n, int h, int w, cudaStream_t st) {
     // the resampling kernels index 16-byte elements in 32 bits
     if ((long long)n * h * w * 16 > INT32_MAX) return dn_fail(RL_INVALID_CALL, "denoiser: %d x %d x %d too large", n, h, w);
     Level L[4];
@@ -1457,7 +1539,7 @@ int forward(rl_denoiser* d, int n, int h, int w, cudaStream_t st) {
         launch_pdl(k_dn_up, dim3(grid_of(tot, 256)), dim3(256), 0, st, in, out, c, L[lvl].w, L[lvl].h, n);
     };
     int rc;
-    if ((rc = conv_fwd(d, 0, d->x, nullptr, L[0].w, L[0].h, n, d->e0, true, st))) return rc;
+    if ((rc = conv_fwd(d, 0, x, nullptr, L[0].w, L[0].h, n, d->e0, true, st))) return rc;
     pool(d->e0, d->p0, 32, 0);
     if ((rc = conv_fwd(d, 1, d->p0, nullptr, L[1].w, L[1].h, n, d->e1, true, st))) return rc;
     pool(d->e1, d->p1, 64, 1);
@@ -1470,12 +1552,12 @@ int forward(rl_denoiser* d, int n, int h, int w, cudaStream_t st) {
     if ((rc = conv_fwd(d, 5, d->u1, d->e1, L[1].w, L[1].h, n, d->d1, true, st))) return rc;
     up(d->d1, d->u0, 64, 0);
     if ((rc = conv_fwd(d, 6, d->u0, d->e0, L[0].w, L[0].h, n, d->d0, true, st))) return rc;
-    if ((rc = conv_fwd(d, 7, d->d0, nullptr, L[0].w, L[0].h, n, d->y, false, st))) return rc;
+    if ((rc = conv_fwd(d, 7, d->d0, nullptr, L[0].w, L[0].h, n, y, false, st))) return rc;
     DN_CK(cudaGetLastError());
     return RL_OK;
 }
 
-int backward(rl_denoiser* d, int n, int h, int w, cudaStream_t st) {
+int backward(rl_denoiser* d, const bf16* x, int n, int h, int w, cudaStream_t st) {
     Level L[4];
     L[0] = {w, h};
     for (int k = 1; k < 4; k++) L[k] = {(L[k - 1].w + 1) / 2, (L[k - 1].h + 1) / 2};
@@ -1517,7 +1599,18 @@ int backward(rl_denoiser* d, int n, int h, int w, cudaStream_t st) {
     if ((rc = conv_dgrad(d, 1, d->ge1, L[1].w, L[1].h, n, d->gp0, nullptr, nullptr, nullptr, st))) return rc;
     pool_bwd(d->gp0, d->e0, d->ge0, 32, 0);
     // encoder e0 = c0(x)
-    if ((rc = conv_wgrad(d, 0, d->ge0, d->x, nullptr, W0, H0, n, st))) return rc;
+    if ((rc = conv_wgrad(d, 0, d->ge0, x, nullptr, W0, H0, n, st))) return rc;
+    LayerGrads G;
+    const bf16* g[8] = {d->ge0, d->ge1, d->ge2, d->ge3, d->gd2, d->gd1, d->gd0, d->gy};
+    const int level[8] = {0, 1, 2, 3, 2, 1, 0, 0};
+    int blocks = 0;
+    for (int l = 0; l < 8; l++) {
+        const Conv& c = d->conv[l];
+        const long long P = (long long)n * L[level[l]].w * L[level[l]].h;
+        G.l[l] = {g[l], c.ncols, c.cout, P, c.gb, blocks};
+        blocks += (int)((P + kBiasPixels - 1) / kBiasPixels);
+    }
+    k_dn_bias_grad<<<blocks, kBiasThreads, 0, st>>>(G);
     DN_CK(cudaGetLastError());
     return RL_OK;
 }
@@ -1699,22 +1792,35 @@ extern "C" int rl_denoiser_train_step(rl_denoiser* d, const void* d_x, const flo
     cudaStream_t st = (cudaStream_t)stream;
     if (int rc = alloc_shapes(d, batch, patch, patch, true, st)) return rc;
     const long long P = (long long)batch * patch * patch;
-    DN_CK(cudaMemcpyAsync(d->x, d_x, P * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
-    DN_CK(cudaMemcpyAsync(d->tgt, d_t, P * sizeof(float4), cudaMemcpyDeviceToDevice, st));
-    // gradient buffers that are accumulated into start at zero
-    if (int rc = forward(d, batch, patch, patch, st)) return rc;
-    k_dn_loss<<<grid_of(P, 256), 256, 0, st>>>(d->y, d->x, d->tgt, P, 1.0f / (float)(P * 3), d->gy, d_loss);
-    if (int rc = backward(d, batch, patch, patch, st)) return rc;
+    // inputs are read where they are, unless a 16-byte load could not
+    const bf16* x = (const bf16*)d_x;
+    const float4* t = (const float4*)d_t;
+    if ((uintptr_t)d_x & 15) {
+        DN_CK(cudaMemcpyAsync(d->x, d_x, P * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
+        x = d->x;
+    }
+    if ((uintptr_t)d_t & 15) {
+        DN_CK(cudaMemcpyAsync(d->tgt, d_t, P * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+        t = d->tgt;
+    }
+    if (int rc = forward(d, x, d->y, batch, patch, patch, st)) return rc;
+    k_dn_loss<<<grid_of(P, 256), 256, 0, st>>>(d->y, x, t, P, 1.0f / (float)(P * 3), d->gy, d_loss);
+    if (int rc = backward(d, x, batch, patch, patch, st)) return rc;
     if (lr < 0.f) return RL_OK;  // gradients only (rl_denoiser_get_grads)
     d->step++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float bc1 = 1.f - powf(b1, (float)d->step), bc2 = 1.f - powf(b2, (float)d->step);
+    LayerSteps A;
+    int blocks = 0;
     for (int l = 0; l < 8; l++) {
         Conv& c = d->conv[l];
-        k_dn_adam<<<grid_of(c.nw(), 256), 256, 0, st>>>(c.w, c.gw, c.mw, c.vw, c.nw(), lr, b1, b2, 1e-8f, bc1, bc2);
-        k_dn_adam<<<1, 128, 0, st>>>(c.b, c.gb, c.mb, c.vb, c.cout, lr, b1, b2, 1e-8f, bc1, bc2);
+        A.l[l] = {c.w, c.gw, c.mw, c.vw, c.b, c.gb, c.mb, c.vb, c.bias, c.wp, c.wt, c.cout, c.ncols, c.segs[0], c.segs[1],
+                  c.kpad, blocks};
+        blocks += (int)((c.nw() + c.cout + kAdamThreads - 1) / kAdamThreads);
     }
-    return pack_all(d, st);
+    k_dn_adam<<<blocks, kAdamThreads, 0, st>>>(A, lr, b1, b2, 1e-8f, bc1, bc2);
+    DN_CK(cudaGetLastError());
+    return RL_OK;
 }
 
 extern "C" int rl_denoiser_apply(rl_denoiser* d, const rl_scene* scene, rl_map* map, const float* d_base,
@@ -1726,7 +1832,7 @@ extern "C" int rl_denoiser_apply(rl_denoiser* d, const rl_scene* scene, rl_map* 
     if (int rc = alloc_shapes(d, 1, m->height, m->width, false, st)) return rc;
     long long n = (long long)m->width * m->height;
     k_dn_features<<<grid_of(n, 256), 256, 0, st>>>(*s, *m, d->x);
-    if (int rc = forward(d, 1, m->height, m->width, st)) return rc;
+    if (int rc = forward(d, d->x, d->y, 1, m->height, m->width, st)) return rc;
     k_dn_apply<<<grid_of(n, 256), 256, 0, st>>>(d->y, d->x, *m, d_base);
     DN_CK(cudaGetLastError());
     return RL_OK;
@@ -1738,9 +1844,18 @@ extern "C" int rl_denoiser_forward(rl_denoiser* d, const void* d_x, int images, 
     cudaStream_t st = (cudaStream_t)stream;
     if (int rc = alloc_shapes(d, images, height, width, d->btrain != 0, st)) return rc;
     const long long P = (long long)images * height * width;
-    DN_CK(cudaMemcpyAsync(d->x, d_x, P * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
-    if (int rc = forward(d, images, height, width, st)) return rc;
-    DN_CK(cudaMemcpyAsync(d_y, d->y, P * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
+    // the first layer reads the caller's features and the last one writes the
+    // caller's output (the features are not read after the first layer, so
+    // the two may be one buffer); copies only where a 16-byte access could not
+    const bf16* x = (const bf16*)d_x;
+    bf16* y = (bf16*)d_y;
+    if ((uintptr_t)d_x & 15) {
+        DN_CK(cudaMemcpyAsync(d->x, d_x, P * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
+        x = d->x;
+    }
+    if ((uintptr_t)d_y & 15) y = d->y;
+    if (int rc = forward(d, x, y, images, height, width, st)) return rc;
+    if (y == d->y) DN_CK(cudaMemcpyAsync(d_y, d->y, P * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
     return RL_OK;
 }
 
