@@ -10,7 +10,7 @@
 //   IndirectLight::bakeLumel           k_indirect_patch (k_indirect, k_indirect_pool: opt-in walks)
 //   RadiosityBuilder form factors      k_ff_pairs, then k_ff_rows + k_ff_scatter + k_ff_finish (CSR)
 //   hemisphere form factors            k_ff_hemi_rays + k_ff_hemi_rle + k_ff_hemi_compact
-//   radiosity gather iterations        k_jacobi4 (k_jacobi_rows per row shard)
+//   radiosity gather iterations        k_jacobi4* (k_jacobi_rows per row shard)
 #include <cuda_runtime.h>
 
 #include <cub/block/block_scan.cuh>
@@ -2489,6 +2489,10 @@ extern "C" int rl_ff_hemisphere_device(const rl_scene* s, int n, const float* d_
 // unused ([n][4], one 16-byte gather, kB = 1).
 template <int kB>
 __device__ __forceinline__ float3 patch_b(const float* __restrict__ B, int c) {
+    if (kB == 3) {  // [n][4], written by the launch before, which may still have been running
+        const float4 v = reinterpret_cast<const float4*>(B)[c];
+        return make_float3(v.x, v.y, v.z);
+    }
     if (kB == 2) {  // [n][3] staged in shared memory
         const float* x = B + 3 * (size_t)c;
         return make_float3(x[0], x[1], x[2]);
@@ -2604,22 +2608,15 @@ __device__ __forceinline__ void row_dot3_quads(int64_t b, int64_t e, int lane, c
 }
 
 // One warp per patch row on [n][4] iterates (w unused), one 16-byte gather
-// per nonzero: B'_i = E_i + rho_i * sum_k F_ik B_k (RGB).  With kQuads,
-// 16-byte column and weight loads as well (a different accumulation order
-// from row_dot3, within the fp32 tolerance).
-template <bool kQuads>
+// per nonzero: B'_i = E_i + rho_i * sum_k F_ik B_k (RGB), for columns or
+// weights that are not 16-byte aligned.
 __global__ void k_jacobi4(int n, const int64_t* row_ptr, const int32_t* cols, const float* vals, const float* E,
                           const float* rho, const float4* B, float4* Bn) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (warp >= n) return;
     float s0, s1, s2;
-    if (kQuads)
-        row_dot3_quads<1>(row_ptr[warp], row_ptr[warp + 1], lane, cols, vals, reinterpret_cast<const float*>(B), s0,
-                          s1, s2);
-    else
-        row_dot3<1>(row_ptr[warp], row_ptr[warp + 1], lane, cols, vals, reinterpret_cast<const float*>(B), s0, s1,
-                    s2);
+    row_dot3<1>(row_ptr[warp], row_ptr[warp + 1], lane, cols, vals, reinterpret_cast<const float*>(B), s0, s1, s2);
     if (lane == 0) {
         size_t i = 3 * (size_t)warp;
         Bn[warp] = make_float4(__fmaf_rn(rho[i], s0, E[i]), __fmaf_rn(rho[i + 1], s1, E[i + 1]),
@@ -2627,14 +2624,184 @@ __global__ void k_jacobi4(int n, const int64_t* row_ptr, const int32_t* cols, co
     }
 }
 
-// k_jacobi4 with the whole iterate staged in shared memory as [n][3] floats
-// (12 n bytes: up to kJacobiSmemPatches patches) by every block, the blocks
-// then taking rows blockIdx.x * warps + warp, + gridDim.x * warps, ...  The
-// column gathers (one per nonzero, scattered over the iterate) then read
-// shared memory instead of 32-byte L2 sectors; the row arithmetic is
-// k_jacobi4's, so the bits are the same.
+// A row of the matrix from the aligned quad that holds its first nonzero on:
+// it is entries [from, to) there, of `limit` that the arrays hold.
+struct RowSpan {
+    const int32_t* cols;
+    const float* vals;
+    int from, to, limit;
+    __device__ __forceinline__ void set(int64_t b, int64_t e, int64_t nnz, const int32_t* c, const float* v) {
+        const int64_t base = b & ~(int64_t)3;
+        cols = c + base;
+        vals = v + base;
+        from = (int)(b - base);
+        to = (int)(e - base);
+        limit = (int)min(nnz - base, (int64_t)INT_MAX);
+    }
+};
+
+// A step of a row: kRowQuads quads of columns and weights per lane; column -1
+// outside the row.  A quad that reaches over the row's ends is read whole and
+// its neighbours' entries are dropped: one path for all lanes, where
+// row_dot3_quads takes a second, entry by entry, at both ends of every row.
+// Only the matrix's last quad may not lie in the arrays.
+constexpr int kRowQuads = 2;
+struct RowStep {
+    int c[kRowQuads][4];
+    float w[kRowQuads][4];
+    __device__ __forceinline__ void load(const RowSpan& r, int base, int lane) {
+#pragma unroll
+        for (int u = 0; u < kRowQuads; u++) {
+            const int q = base + 128 * u + 4 * lane;
+            int4 cc = make_int4(-1, -1, -1, -1);
+            float4 ww = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (q < r.to) {
+                if (q + 4 <= r.limit) {
+                    cc = __ldg(reinterpret_cast<const int4*>(r.cols + q));
+                    ww = __ldg(reinterpret_cast<const float4*>(r.vals + q));
+                } else {
+                    cc.x = __ldg(r.cols + q);
+                    ww.x = __ldg(r.vals + q);
+                    if (q + 1 < r.limit) { cc.y = __ldg(r.cols + q + 1); ww.y = __ldg(r.vals + q + 1); }
+                    if (q + 2 < r.limit) { cc.z = __ldg(r.cols + q + 2); ww.z = __ldg(r.vals + q + 2); }
+                }
+            }
+            c[u][0] = cc.x; c[u][1] = cc.y; c[u][2] = cc.z; c[u][3] = cc.w;
+            w[u][0] = ww.x; w[u][1] = ww.y; w[u][2] = ww.z; w[u][3] = ww.w;
+        }
+    }
+    // row_dot3_quads' terms in its order: quads alternate between two sums
+    template <int kB>
+    __device__ __forceinline__ void add(const RowSpan& r, int base, int lane, const float* __restrict__ B,
+                                        float (&s)[2][3]) const {
+#pragma unroll
+        for (int u = 0; u < kRowQuads; u++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int q = base + 128 * u + 4 * lane + j;
+                if (q >= r.from && q < r.to) {
+                    const float3 x = patch_b<kB>(B, c[u][j]);
+                    s[u & 1][0] = __fmaf_rn(w[u][j], x.x, s[u & 1][0]);
+                    s[u & 1][1] = __fmaf_rn(w[u][j], x.y, s[u & 1][1]);
+                    s[u & 1][2] = __fmaf_rn(w[u][j], x.z, s[u & 1][2]);
+                }
+            }
+    }
+};
+
+// Row `row` of Bn from its sums: lane c < 3 writes channel c.
+__device__ __forceinline__ void row_finish(const float (&s)[2][3], int lane, float e, float rho, float4* Bn, int row) {
+    float r0 = s[0][0] + s[1][0], r1 = s[0][1] + s[1][1], r2 = s[0][2] + s[1][2];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        r0 += __shfl_xor_sync(0xffffffffu, r0, o);
+        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+        r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+    }
+    if (lane < 4)
+        reinterpret_cast<float*>(Bn + row)[lane] =
+            lane < 3 ? __fmaf_rn(rho, lane == 0 ? r0 : lane == 1 ? r1 : r2, e) : 0.f;
+}
+
+// k_jacobi4's step with the whole iterate staged in shared memory as [n][3]
+// floats (12 n bytes: up to kJacobiSmemPatches patches) by every block, the
+// blocks then taking rows blockIdx.x * warps + warp, + gridDim.x * warps, ...
+// The column gathers (one per nonzero, scattered over the iterate) then read
+// shared memory instead of 32-byte L2 sectors; 3.5 lanes share a bank, which
+// makes them half the kernel's time.  Each row's first loads run while the row
+// before is reduced, and the kernel is launched while its predecessor ends
+// (programmatic dependent launch), which is most of what a small system
+// spends.  50 iterations: 16,384 patches with 7.3 M nonzeros 1,247 us with
+// row_dot3_quads and full launches, 1,085 us so; 4,096 patches with 0.9 M 425
+// -> 244 us; 1,024 patches 320 -> 157 us.  Four quads a step (1,116 us) and
+// the next step's loads before this one's sums (1,319 us) need more registers
+// than 32 warps have.
 constexpr int kJacobiSmemPatches = (224 * 1024) / 12;
-template <bool kQuads>
+__global__ void __launch_bounds__(1024, 1) k_jacobi4_quads_smem(int n, const int64_t* __restrict__ row_ptr,
+                                                                const int32_t* __restrict__ cols,
+                                                                const float* __restrict__ vals, const float* E,
+                                                                const float* rho, const float4* B, float4* Bn) {
+    extern __shared__ float sb[];
+    const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+    const int stride = gridDim.x * warps;
+    int row = blockIdx.x * warps + (threadIdx.x >> 5);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the matrix is older than the iterate: its first rows are read before the wait
+    const int64_t nnz = row_ptr[n];
+    RowSpan span;
+    RowStep step;
+    if (row < n) {
+        span.set(row_ptr[row], row_ptr[row + 1], nnz, cols, vals);
+        step.load(span, 0, lane);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const float4 v = B[i];
+        sb[3 * i] = v.x;
+        sb[3 * i + 1] = v.y;
+        sb[3 * i + 2] = v.z;
+    }
+    __syncthreads();
+    while (row < n) {
+        const int next = row + stride;
+        int64_t nb = 0, ne = 0;
+        if (next < n) {
+            nb = row_ptr[next];
+            ne = row_ptr[next + 1];
+        }
+        float er = 0.f, rr = 0.f;
+        if (lane < 3) {
+            er = E[3 * (size_t)row + lane];
+            rr = rho[3 * (size_t)row + lane];
+        }
+        float s[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        for (int base = 0;;) {
+            step.add<2>(span, base, lane, sb, s);
+            base += 128 * kRowQuads;
+            if (base >= span.to) break;
+            step.load(span, base, lane);
+        }
+        if (next < n) {  // the next row's loads run while this one is reduced
+            span.set(nb, ne, nnz, cols, vals);
+            step.load(span, 0, lane);
+        }
+        row_finish(s, lane, er, rr, Bn, row);
+        row = next;
+    }
+}
+
+// The same without the staging, for iterates that do not fit: one warp per
+// row, one 16-byte gather per nonzero.  25,600 patches, 50 iterations: 2,160
+// -> 1,874 us.
+__global__ void __launch_bounds__(256) k_jacobi4_quads(int n, const int64_t* __restrict__ row_ptr,
+                                                       const int32_t* __restrict__ cols,
+                                                       const float* __restrict__ vals, const float* E, const float* rho,
+                                                       const float4* B, float4* Bn) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (row >= n) return;
+    RowSpan span;
+    RowStep step;
+    span.set(row_ptr[row], row_ptr[row + 1], row_ptr[n], cols, vals);
+    step.load(span, 0, lane);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float er = 0.f, rr = 0.f;
+    if (lane < 3) {
+        er = E[3 * (size_t)row + lane];
+        rr = rho[3 * (size_t)row + lane];
+    }
+    float s[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    for (int base = 0;;) {
+        step.add<3>(span, base, lane, reinterpret_cast<const float*>(B), s);
+        base += 128 * kRowQuads;
+        if (base >= span.to) break;
+        step.load(span, base, lane);
+    }
+    row_finish(s, lane, er, rr, Bn, row);
+}
+
+// k_jacobi4 with the whole iterate staged in shared memory (as
+// k_jacobi4_quads_smem), for columns or weights that are not 16-byte aligned.
 __global__ void __launch_bounds__(1024, 1) k_jacobi4_smem(int n, const int64_t* row_ptr, const int32_t* cols,
                                                           const float* vals, const float* E, const float* rho,
                                                           const float4* B, float4* Bn) {
@@ -2649,10 +2816,7 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi4_smem(int n, const int64_t* 
     const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
     for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < n; row += gridDim.x * warps) {
         float s0, s1, s2;
-        if (kQuads)
-            row_dot3_quads<2>(row_ptr[row], row_ptr[row + 1], lane, cols, vals, sb, s0, s1, s2);
-        else
-            row_dot3<2>(row_ptr[row], row_ptr[row + 1], lane, cols, vals, sb, s0, s1, s2);
+        row_dot3<2>(row_ptr[row], row_ptr[row + 1], lane, cols, vals, sb, s0, s1, s2);
         if (lane == 0) {
             size_t i = 3 * (size_t)row;
             Bn[row] = make_float4(__fmaf_rn(rho[i], s0, E[i]), __fmaf_rn(rho[i + 1], s1, E[i + 1]),
@@ -2661,40 +2825,40 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi4_smem(int n, const int64_t* 
     }
 }
 
+// Whether launches on `st` may overlap their predecessors' ends: not in a
+// graph that is being captured, whose nodes keep full dependencies.
+static bool may_overlap(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+}
+
 // One Jacobi step of rl_radiosity_solve (and its no-allocation form): the
-// shared-memory kernel when the iterate fits, else k_jacobi4.
+// shared-memory kernels when the iterate fits, else k_jacobi4.  `overlap`: the launch may start while its predecessor, a kernel
+// of the same solve, is ending.
 static int jacobi4_step(int n, const int64_t* row_ptr, const int32_t* cols, const float* vals, const float* E,
-                 const float* rho, const float4* B, float4* Bn, cudaStream_t st) {
+                 const float* rho, const float4* B, float4* Bn, bool overlap, cudaStream_t st) {
     const bool quads = ((uintptr_t)cols % 16) == 0 && ((uintptr_t)vals % 16) == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks_for((long long)n * 32, 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = quads && overlap ? 1 : 0;  // the other kernels do not wait for their predecessor themselves
+    auto kernel = quads ? k_jacobi4_quads : k_jacobi4;
     if (n <= kJacobiSmemPatches) {
-        static int sms = 0;
-        static std::once_flag once;
-        cudaError_t ae = cudaSuccess;
-        std::call_once(once, [&] {
-            ae = cudaFuncSetAttribute(k_jacobi4_smem<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (ae == cudaSuccess)
-                ae = cudaFuncSetAttribute(k_jacobi4_smem<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          227 * 1024);
-            int dev = 0;
-            if (ae == cudaSuccess) ae = cudaGetDevice(&dev);
-            if (ae == cudaSuccess) ae = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        });
-        if (ae != cudaSuccess) return fail(RL_CUDA_ERROR, "jacobi set-up: %s", cudaGetErrorString(ae));
-        const int grid = std::max(1, std::min(sms, (n + 31) / 32));
-        const size_t smem = 12 * (size_t)n;
-        if (quads)
-            k_jacobi4_smem<true><<<grid, 1024, smem, st>>>(n, row_ptr, cols, vals, E, rho, B, Bn);
-        else
-            k_jacobi4_smem<false><<<grid, 1024, smem, st>>>(n, row_ptr, cols, vals, E, rho, B, Bn);
-        CK_LAUNCH("k_jacobi4_smem");
-        return RL_OK;
+        int dev = 0, sms = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        kernel = quads ? k_jacobi4_quads_smem : k_jacobi4_smem;
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        cfg.gridDim = dim3((unsigned)std::max(1, std::min(sms, (n + 31) / 32)));
+        cfg.blockDim = dim3(1024);
+        cfg.dynamicSmemBytes = 12 * (size_t)n;
     }
-    const unsigned grid = blocks_for((long long)n * 32, 256);
-    if (quads)
-        k_jacobi4<true><<<grid, 256, 0, st>>>(n, row_ptr, cols, vals, E, rho, B, Bn);
-    else
-        k_jacobi4<false><<<grid, 256, 0, st>>>(n, row_ptr, cols, vals, E, rho, B, Bn);
-    CK_LAUNCH("k_jacobi4");
+    CK(cudaLaunchKernelEx(&cfg, kernel, n, row_ptr, cols, vals, E, rho, B, Bn));
     return RL_OK;
 }
 
@@ -2772,8 +2936,9 @@ extern "C" int rl_radiosity_solve(int n, const int64_t* d_row_ptr, const int32_t
     if (rc) return rc;
     k_pack4<<<blocks_for(n, 256), 256, 0, st>>>(n, d_E, src);
     CK_LAUNCH("k_pack4");
+    const bool overlap = may_overlap(st);
     for (int it = 0; it < iters; it++) {
-        if (int rc2 = jacobi4_step(n, d_row_ptr, d_cols, d_vals, d_E, d_rho, src, dst, st)) return rc2;
+        if (int rc2 = jacobi4_step(n, d_row_ptr, d_cols, d_vals, d_E, d_rho, src, dst, overlap, st)) return rc2;
         std::swap(src, dst);
     }
     k_unpack4<<<blocks_for(n, 256), 256, 0, st>>>(n, src, d_B);
@@ -3600,8 +3765,9 @@ extern "C" int rl_radiosity_solve_noalloc(int n, const int64_t* d_row_ptr, const
     float4* dst = scratch_base + RL_SOLVE_NOALLOC_MAX_PATCHES;
     k_pack4<<<blocks_for(n, 256), 256, 0, st>>>(n, d_E, src);
     CK_LAUNCH("k_pack4");
+    const bool overlap = may_overlap(st);
     for (int it = 0; it < iters; it++) {
-        if (int rc2 = jacobi4_step(n, d_row_ptr, d_cols, d_vals, d_E, d_rho, src, dst, st)) return rc2;
+        if (int rc2 = jacobi4_step(n, d_row_ptr, d_cols, d_vals, d_E, d_rho, src, dst, overlap, st)) return rc2;
         std::swap(src, dst);
     }
     k_unpack4<<<blocks_for(n, 256), 256, 0, st>>>(n, src, d_B);
