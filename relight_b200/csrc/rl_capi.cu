@@ -2120,20 +2120,50 @@ __global__ void k_ff_finish(int n, const long long* row_ptr, const int2* entries
 }
 
 namespace {
-// Pinned host memory of the calling thread for small results: a copy into it
-// does not wait, one into pageable memory does (about 10 us each).
+// Pinned host memory for small results: a copy into it does not wait, one
+// into pageable memory does (about 10 us each).  A call takes one block from a
+// few that the process keeps, or pins its own when they are all out (about a
+// millisecond); a block that a failed call may still have a copy in flight to
+// is not kept.
 struct PinnedStaging {
-    static constexpr size_t kBytes = 1 << 20;
+    static constexpr size_t kBytes = 1 << 20, kKept = 4;
     char* p = nullptr;
+    bool settled = true;   // no copy in flight
     int reserve() {
+        {
+            std::lock_guard<std::mutex> lk(mutex());
+            if (!kept().empty()) {
+                p = kept().back();
+                kept().pop_back();
+            }
+        }
         if (!p) CK(cudaMallocHost((void**)&p, kBytes));
+        settled = false;
         return RL_OK;
     }
     ~PinnedStaging() {
-        if (p) cudaFreeHost(p);
+        if (!p) return;
+        if (settled) {
+            std::lock_guard<std::mutex> lk(mutex());
+            if (kept().size() < kKept) {
+                kept().push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);   // waits for the device
+    }
+
+   private:
+    static std::mutex& mutex() {
+        static std::mutex mu;
+        return mu;
+    }
+    static std::vector<char*>& kept() {
+        static std::vector<char*>* blocks = new std::vector<char*>;   // outlives the last call at exit
+        if (blocks->capacity() < kKept) blocks->reserve(kKept);
+        return *blocks;
     }
 };
-thread_local PinnedStaging t_pinned;
 }  // namespace
 
 extern "C" int rl_ff_pairwise(const rl_scene* s, int n, const float* d_pos, const float* d_nrm, float threshold,
@@ -2144,7 +2174,7 @@ extern "C" int rl_ff_pairwise(const rl_scene* s, int n, const float* d_pos, cons
     // one block for the sweep ([counter, rows' counts and cursors, pairs]) and
     // one for the CSR ([row_ptr, columns, values, unordered entries]); small
     // results come back through pinned memory in one copy each
-    PinnedStaging& pin = t_pinned;
+    PinnedStaging pin;
     if (int rc = pin.reserve()) return rc;
     const size_t rows = (size_t)std::max(n, 1), heads = 1 + rows;
     Scratch sweep, csr;
@@ -2169,9 +2199,11 @@ extern "C" int rl_ff_pairwise(const rl_scene* s, int n, const float* d_pos, cons
                                                       s->d_status);
             CK_LAUNCH("k_ff_pairs");
         }
+        pin.settled = false;
         CK(cudaMemcpyAsync(pin.p, counter, 8, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(pin.p + 8, s->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        pin.settled = true;
         std::memcpy(&found, pin.p, 8);
         std::memcpy(&flags, pin.p + 8, sizeof(int));
         if (found <= cap) break;
@@ -2200,9 +2232,11 @@ extern "C" int rl_ff_pairwise(const rl_scene* s, int n, const float* d_pos, cons
         CK_LAUNCH("k_ff_finish");
     }
     if (rp + 2 * part <= PinnedStaging::kBytes) {
+        pin.settled = false;
         CK(cudaMemcpyAsync(pin.p, drow, rp, cudaMemcpyDeviceToHost, st));
         if (count) CK(cudaMemcpyAsync(pin.p + rp, dcols, 2 * part, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        pin.settled = true;
         std::memcpy(row_ptr, pin.p, rp);
         std::memcpy(cols, pin.p + rp, part);
         std::memcpy(vals, pin.p + rp + part, part);
@@ -2381,7 +2415,7 @@ static int ff_hemisphere(const rl_scene* s, int n, const float* d_pos, const flo
             return fail(RL_INVALID_CALL, "rl_ff_hemisphere: map %d outside patch_of_texel", m);
     // one block for the tables (the caller's, uploaded in one copy when they
     // fit in pinned memory), one for hits, runs and rows
-    PinnedStaging& pin = t_pinned;
+    PinnedStaging pin;
     if (int rc = pin.reserve()) return rc;
     const size_t nm = (size_t)std::max(nmaps, 1);
     const size_t at_dims = 8 * nm, at_mesh = at_dims + 8 * nm, at_pot = at_mesh + 4 * (size_t)s->nmeshes,
@@ -2434,6 +2468,7 @@ static int ff_hemisphere(const rl_scene* s, int n, const float* d_pos, const flo
     CK(cudaMemcpyAsync(pin.p, drow + n, 8, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(pin.p + 8, s->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    pin.settled = true;
     int64_t total_nnz = 0;
     int flags = 0;
     std::memcpy(&total_nnz, pin.p, 8);
