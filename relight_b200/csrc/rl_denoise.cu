@@ -669,118 +669,147 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 
 // ------------------------------------------------- the weight gradient
 
-struct WgradArgs {
-    int W, H, N;           // spatial size, images
-    int tiles_x, tiles_y;  // pixel tiles per image
-    int splits;            // CTAs sharing the pixel range of one (tap, chunk)
-    int nb;                // 64-channel input blocks in this launch (N = 64 nb)
-    int c_base;            // first input channel of this launch
+// dW[co][tap][ci] += sum over pixels p of G[p][co] * X[p + off(tap)][ci].
+// GEMM with M = 128 gradient channels (the rows past cout are not kept),
+// N = up to 64 input channels, K = pixels; both operands are the NHWC boxes as
+// stored, i.e. MN-major.  One launch takes a list of such products (all
+// layers of the network); a CTA takes one product, one row of three taps and a
+// share of the pixel tiles.
+//
+// What bounds it: an issuing thread spends about 150 cycles on each MMA
+// whatever its N, 8 a tile and tap, so each of the three taps has its own
+// issuing warp and accumulator and reads the same G tile.  One tap per CTA
+// read G nine times and had one issuer, and a launch per layer and segment
+// left most of the chip idle on the small layers: 16 patches of 64 x 64,
+// 278 us in 11 launches, 57 us in one.
+constexpr int kWgItems = 16, kWgTaps = 3, kWgCols = 64;
+
+struct WgradItem {
+    int tiles_x, tiles_y, tiles;  // pixel tiles per image, in all images
+    int cta0, splits;      // CTAs [cta0, cta0 + 3 splits): tap row x split
+    int n;                 // MMA N: input channels of this item, up to 16s
+    int c_base;            // first input channel
     int cin;               // input channels of the segment (columns written: c_base + c < cin)
     int cout;              // gradient channels (rows written)
     int ci_off;            // column offset of the segment in dW
     int ci_total;          // dW row length per tap
-    int stages;
     float* dw;             // [cout][9][ci_total], accumulated with atomics
+};
+struct WgradList {
+    CUtensorMap g[kWgItems], x[kWgItems];
+    WgradItem item[kWgItems];
+    int items;
     int* err;
 };
 
-// dW[co][tap][ci] += sum over pixels p of G[p][co] * X[p + off(tap)][ci].
-// GEMM with M = 128 gradient channels (the second 64 read as zeros when
-// absent), N = 64 nb input channels, K = pixels; both operands are the
-// NHWC boxes as stored, i.e. MN-major.  grid = (9 taps, 1, splits); one
-// launch covers input channels [c_base, c_base + 64 nb).
-__global__ void __launch_bounds__(128, 1) k_conv3x3_wgrad(const __grid_constant__ CUtensorMap tmG,
-                                                         const __grid_constant__ CUtensorMap tmX, const WgradArgs a) {
+constexpr int kWgStagesMax = 3;
+__host__ __device__ constexpr uint32_t wgrad_stage_bytes(int cout) {
+    return (uint32_t)((cout > 64 ? 2 : 1) + kWgTaps) * kABytes;
+}
+__host__ __device__ constexpr int wgrad_stages(int cout) { return cout > 64 ? 2 : 3; }
+constexpr uint32_t kWgSmem = 3 * wgrad_stage_bytes(64) + 1024 + 128;
+static_assert(2 * wgrad_stage_bytes(128) <= 3 * wgrad_stage_bytes(64), "both splits fit");
+
+__global__ void __launch_bounds__(128, 1) k_conv3x3_wgrad(const __grid_constant__ WgradList L) {
     extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t full[kWgStagesMax], empty[kWgStagesMax], done;
+    __shared__ uint32_t tmem_slot;
     uint8_t* smem = align1024(smem_raw);
-    const int S = a.stages;
-    const uint32_t a_bytes = 2 * kABytes;
-    const uint32_t b_bytes = (uint32_t)a.nb * kABytes;
-    uint8_t* sa = smem;
-    uint8_t* sb = smem + S * a_bytes;
-    uint64_t* full = (uint64_t*)(sb + S * b_bytes);
-    uint64_t* empty = full + S;
-    uint64_t* done = empty + S;
-    uint32_t* tmem_slot = (uint32_t*)(done + 1);
+    int which = 0;
+    while (which + 1 < L.items && (int)blockIdx.x >= L.item[which + 1].cta0) which++;
+    const WgradItem& a = L.item[which];
+    const int unit = (int)blockIdx.x - a.cta0;
+    const int dy = unit % 3 - 1, split = unit / 3;
+    const bool wide = a.cout > 64;
+    const int S = wgrad_stages(a.cout);
+    const uint32_t stage_bytes = wgrad_stage_bytes(a.cout), g_bytes = wide ? 2 * kABytes : kABytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tap = blockIdx.x, split = blockIdx.z;
-    const int n = a.nb * 64;
-    const uint32_t tcols = n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; s++) {
             mbar_init(full + s, 1);
-            mbar_init(empty + s, 1);
+            mbar_init(empty + s, kWgTaps);
         }
-        mbar_init(done, 1);
+        mbar_init(&done, kWgTaps);
         fence_barrier_init();
     }
     if (warp == 0) {
-        tmem_alloc(tmem_slot, tcols);
+        tmem_alloc(&tmem_slot, 256);
         tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const long long tiles = (long long)a.tiles_x * a.tiles_y * a.N;
-    const long long mine = tiles > split ? (tiles - split + a.splits - 1) / a.splits : 0;
-    const int dx = tap % 3 - 1, dy = tap / 3 - 1;
+    const uint32_t tmem = tmem_slot;
+    const int mine = a.tiles > split ? (a.tiles - split + a.splits - 1) / a.splits : 0;
 
     if (warp == 0 && lane == 0) {
-        long long issued = 0;
-        for (long long kb = 0; kb < mine; kb++) {
-            const int s = (int)(kb % S);
-            const long long round = kb / S;
-            if (!mbar_wait(empty + s, (uint32_t)((round & 1) ^ 1), a.err, 8)) break;
+        int issued = 0;
+        for (int kb = 0; kb < mine; kb++) {
+            const int s = kb % S;
+            if (!mbar_wait(empty + s, (uint32_t)(((kb / S) & 1) ^ 1), L.err, 8)) break;
             issued = kb + 1;
-            const long long t = split + kb * a.splits;
-            const int tx = (int)(t % a.tiles_x), ty = (int)((t / a.tiles_x) % a.tiles_y), img = (int)(t / ((long long)a.tiles_x * a.tiles_y));
-            const int x0 = tx * kTileW, y0 = ty * kTileH;
-            mbar_expect_tx(full + s, a_bytes + b_bytes);
-            tma_load_4d(sa + s * a_bytes, &tmG, full + s, 0, x0, y0, img);
-            tma_load_4d(sa + s * a_bytes + kABytes, &tmG, full + s, 64, x0, y0, img);
-            for (int j = 0; j < a.nb; j++)
-                tma_load_4d(sb + s * b_bytes + j * kABytes, &tmX, full + s, a.c_base + j * 64, x0 + dx, y0 + dy, img);
+            const int t = split + kb * a.splits;
+            const int row = t / a.tiles_x, img = row / a.tiles_y;
+            const int x0 = (t - row * a.tiles_x) * kTileW, y0 = (row - img * a.tiles_y) * kTileH;
+            uint8_t* st = smem + s * stage_bytes;
+            mbar_expect_tx(full + s, stage_bytes);
+            tma_load_4d(st, &L.g[which], full + s, 0, x0, y0, img);
+            if (wide) tma_load_4d(st + kABytes, &L.g[which], full + s, 64, x0, y0, img);
+            for (int j = 0; j < kWgTaps; j++)
+                tma_load_4d(st + g_bytes + j * kABytes, &L.x[which], full + s, a.c_base, x0 + j - 1, y0 + dy, img);
         }
-        for (long long kb = issued > S ? issued - S : 0; kb < issued; kb++)
-            mbar_wait(full + kb % S, (uint32_t)((kb / S) & 1), a.err, 64);
-    } else if (warp == 1 && lane == 0) {
-        const uint32_t idesc = idesc_bf16(n, true, true);
-        for (long long kb = 0; kb < mine; kb++) {
-            const int s = (int)(kb % S);
-            const long long round = kb / S;
-            if (!mbar_wait(full + s, (uint32_t)(round & 1), a.err, 16)) break;
+        for (int kb = issued > S ? issued - S : 0; kb < issued; kb++)
+            mbar_wait(full + kb % S, (uint32_t)((kb / S) & 1), L.err, 64);
+    } else if (warp > 0 && lane == 0) {
+        const uint32_t idesc = idesc_bf16(a.n, true, true);
+        const uint32_t d = tmem + (uint32_t)((warp - 1) * kWgCols);
+        for (int kb = 0; kb < mine; kb++) {
+            const int s = kb % S;
+            if (!mbar_wait(full + s, (uint32_t)((kb / S) & 1), L.err, 16)) break;
             tc_fence_after();
-            // MN-major: 64-element blocks along M / N are 16 KB apart (LBO),
-            // groups of 8 pixel rows 1 KB apart (SBO); K = 16 pixels per MMA.
-            const uint32_t abase = smem_u32(sa + s * a_bytes), bbase = smem_u32(sb + s * b_bytes);
+            // MN-major: 64-element blocks along M are 16 KB apart (LBO; up to
+            // 64 gradient channels the second block is the first tap's X tile,
+            // and its rows are not kept), groups of 8 pixel rows 1 KB apart
+            // (SBO); K = 16 pixels per MMA.
+            const uint32_t abase = smem_u32(smem + s * stage_bytes);
+            const uint32_t bbase = abase + g_bytes + (uint32_t)(warp - 1) * kABytes;
 #pragma unroll
             for (int kk = 0; kk < 8; kk++)
-                umma_bf16(tmem, desc_sw128(abase + kk * 2048, kABytes, 1024), desc_sw128(bbase + kk * 2048, kABytes, 1024),
+                umma_bf16(d, desc_sw128(abase + kk * 2048, kABytes, 1024), desc_sw128(bbase + kk * 2048, kABytes, 1024),
                           idesc, (kb | kk) != 0);
             umma_commit(empty + s);
         }
-        umma_commit(done);
+        umma_commit(&done);
     }
     __syncwarp();
 
-    const bool finished = mbar_wait(done, 0, a.err, 32) && mine > 0;
+    const bool finished = mbar_wait(&done, 0, L.err, 32) && mine > 0;
     tc_fence_after();
     const int co = warp * 32 + lane;
-    for (int c = 0; c < n; c += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, r);
-        if (!finished || co >= a.cout) continue;
-        const int ci0 = a.c_base + c;
-        float* dst = a.dw + ((long long)co * 9 + tap) * a.ci_total + a.ci_off;
+    if (warp * 32 < a.cout)
+        for (int j = 0; j < kWgTaps; j++)
+            for (int c = 0; c < a.n; c += 16) {
+                uint32_t r[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * kWgCols + c), r);
+                if (!finished || co >= a.cout) continue;
+                const int ci0 = a.c_base + c;
+                float* dst = a.dw + ((long long)co * 9 + 3 * (dy + 1) + j) * a.ci_total + a.ci_off + ci0;
+                if (ci0 + 16 <= a.cin && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
-        for (int i = 0; i < 16; i++)
-            if (ci0 + i < a.cin) atomicAdd(dst + ci0 + i, __uint_as_float(r[i]));
-    }
+                    for (int i = 0; i < 16; i += 4)
+                        atomicAdd(reinterpret_cast<float4*>(dst + i),
+                                  make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]),
+                                              __uint_as_float(r[i + 3])));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        if (ci0 + i < a.cin) atomicAdd(dst + i, __uint_as_float(r[i]));
+                }
+            }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, tcols);
+    if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
 // Launch with programmatic stream serialisation (see pdl_wait).
@@ -983,48 +1012,87 @@ extern "C" int rl_dn_conv3x3(const void* in0, int c0, const void* in1, int c1, i
     return RL_OK;
 }
 
+namespace {
+
+// The products of one k_conv3x3_wgrad launch.
+struct WgradBatch {
+    WgradList list;
+    cudaStream_t st;
+
+    WgradBatch(int* d_err, cudaStream_t stream) : st(stream) {
+        list.items = 0;
+        list.err = d_err;
+    }
+
+    int add(const void* grad, int cout, int grad_cs, const void* in, int cin, int in_cs, int width, int height,
+            int images, float* dw, int ci_off, int ci_total) {
+        for (int c = 0; c < cin; c += kWgCols) {
+            if (list.items == kWgItems)
+                if (int rc = launch()) return rc;
+            if (int rc = act_map(&list.g[list.items], grad, grad_cs, width, height, images)) return rc;
+            if (int rc = act_map(&list.x[list.items], in, in_cs, width, height, images)) return rc;
+            WgradItem& a = list.item[list.items++];
+            a.tiles_x = (width + kTileW - 1) / kTileW;
+            a.tiles_y = (height + kTileH - 1) / kTileH;
+            a.tiles = a.tiles_x * a.tiles_y * images;
+            a.splits = 1;
+            a.n = std::min(kWgCols, (cin - c + 15) / 16 * 16);
+            a.c_base = c;
+            a.cin = cin;
+            a.cout = cout;
+            a.ci_off = ci_off;
+            a.ci_total = ci_total;
+            a.dw = dw;
+        }
+        return RL_OK;
+    }
+
+    // Shares out one CTA per SM (three to each split of an item's tiles): the
+    // next split goes to the item whose CTAs have the most tiles.
+    int launch() {
+        if (list.items == 0) return RL_OK;
+        static std::once_flag attr;
+        static cudaError_t ae = cudaSuccess;
+        static int sms = 148;
+        std::call_once(attr, [] {
+            ae = cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
+            int dev = 0;
+            if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        });
+        if (ae != cudaSuccess) return dn_fail(RL_CUDA_ERROR, "wgrad smem attribute: %s", cudaGetErrorString(ae));
+        for (int left = sms / 3 - list.items; left > 0; left--) {
+            WgradItem* most = &list.item[0];
+            for (int i = 1; i < list.items; i++)
+                if ((long long)list.item[i].tiles * most->splits > (long long)most->tiles * list.item[i].splits)
+                    most = &list.item[i];
+            if (most->splits >= most->tiles) break;
+            most->splits++;
+        }
+        int ctas = 0;
+        for (int i = 0; i < list.items; i++) {
+            list.item[i].cta0 = ctas;
+            ctas += 3 * list.item[i].splits;
+        }
+        k_conv3x3_wgrad<<<ctas, 128, kWgSmem, st>>>(list);
+        cudaError_t e = cudaGetLastError();
+        list.items = 0;
+        if (e != cudaSuccess) return dn_fail(RL_CUDA_ERROR, "k_conv3x3_wgrad: %s", cudaGetErrorString(e));
+        return RL_OK;
+    }
+};
+
+}  // namespace
+
 extern "C" int rl_dn_conv3x3_wgrad(const void* grad, int cout, int grad_cs, const void* in, int cin, int in_cs,
                                    int width, int height, int images, float* dw, int ci_off, int ci_total, int* d_err,
                                    void* stream) {
     if (!grad || !in || !dw || cout <= 0 || cout > 128 || cin <= 0 || width <= 0 || height <= 0 || images <= 0)
         return dn_fail(RL_INVALID_CALL, "rl_dn_conv3x3_wgrad: bad arguments");
-    CUtensorMap tG, tX;
-    if (int rc = act_map(&tG, grad, grad_cs, width, height, images)) return rc;
-    if (int rc = act_map(&tX, in, in_cs, width, height, images)) return rc;
-    const int blocks = (cin + 63) / 64, chunks = (blocks + 3) / 4;
-    WgradArgs a;
-    memset(&a, 0, sizeof a);
-    a.W = width;
-    a.H = height;
-    a.N = images;
-    a.tiles_x = (width + kTileW - 1) / kTileW;
-    a.tiles_y = (height + kTileH - 1) / kTileH;
-    a.cin = cin;
-    a.cout = cout;
-    a.ci_off = ci_off;
-    a.ci_total = ci_total;
-    a.dw = dw;
-    a.err = d_err;
-    static std::once_flag attr;
-    cudaError_t ae = cudaSuccess;
-    std::call_once(attr, [&] {
-        ae = cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    });
-    if (ae != cudaSuccess) return dn_fail(RL_CUDA_ERROR, "wgrad smem attribute: %s", cudaGetErrorString(ae));
-    const long long tiles = (long long)a.tiles_x * a.tiles_y * images;
-    const int splits = (int)std::min<long long>(tiles, 32);
-    for (int ch = 0; ch < chunks; ch++) {
-        WgradArgs b = a;
-        b.nb = std::min(4, blocks - ch * 4);
-        b.c_base = ch * 256;
-        b.stages = b.nb > 2 ? 2 : 3;
-        b.splits = splits;
-        const int smem = b.stages * (int)(2 * kABytes + b.nb * kABytes) + 2 * b.stages * 8 + 16 + 1024;
-        k_conv3x3_wgrad<<<dim3(9, 1, splits), 128, smem, (cudaStream_t)stream>>>(tG, tX, b);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return dn_fail(RL_CUDA_ERROR, "k_conv3x3_wgrad: %s", cudaGetErrorString(e));
-    }
-    return RL_OK;
+    if ((long long)((width + kTileW - 1) / kTileW) * ((height + kTileH - 1) / kTileH) * images > INT32_MAX)
+        return dn_fail(RL_INVALID_CALL, "rl_dn_conv3x3_wgrad: too many tiles");
+    WgradBatch b(d_err, (cudaStream_t)stream);
+    if (int rc = b.add(grad, cout, grad_cs, in, cin, in_cs, width, height, images, dw, ci_off, ci_total)) return rc;
+    return b.launch();
 }
 
 // ================================================================ network
@@ -1509,17 +1577,11 @@ int conv_dgrad(rl_denoiser* d, int l, const bf16* gout, int w, int h, int n, bf1
                          c.segs[0], m0, g1, pad64(c.segs[0]), g1 ? c.segs[1] : 0, g1 ? c.segs[1] : 0, m1, d->d_err, st);
 }
 
-int conv_wgrad(rl_denoiser* d, int l, const bf16* gout, const bf16* in0, const bf16* in1, int w, int h, int n,
-               cudaStream_t st) {
+int conv_wgrad(rl_denoiser* d, WgradBatch& b, int l, const bf16* gout, const bf16* in0, const bf16* in1, int w, int h,
+               int n) {
     Conv& c = d->conv[l];
-    if (int rc = rl_dn_conv3x3_wgrad(gout, c.cout, c.ncols, in0, c.segs[0], c.segs[0], w, h, n, c.gw, 0, c.kpad,
-                                     d->d_err, st))
-        return rc;
-    if (in1)
-        if (int rc = rl_dn_conv3x3_wgrad(gout, c.cout, c.ncols, in1, c.segs[1], c.segs[1], w, h, n, c.gw,
-                                         pad64(c.segs[0]), c.kpad, d->d_err, st))
-            return rc;
-    return RL_OK;
+    if (int rc = b.add(gout, c.cout, c.ncols, in0, c.segs[0], c.segs[0], w, h, n, c.gw, 0, c.kpad)) return rc;
+    return in1 ? b.add(gout, c.cout, c.ncols, in1, c.segs[1], c.segs[1], w, h, n, c.gw, pad64(c.segs[0]), c.kpad) : RL_OK;
 }
 
 // x and y: the network's input and output, the denoiser's own buffers or the
@@ -1572,34 +1634,37 @@ int backward(rl_denoiser* d, const bf16* x, int n, int h, int w, cudaStream_t st
     int rc;
     const int W0 = L[0].w, H0 = L[0].h;
     // output layer
-    if ((rc = conv_wgrad(d, 7, d->gy, d->d0, nullptr, W0, H0, n, st))) return rc;
     if ((rc = conv_dgrad(d, 7, d->gy, W0, H0, n, d->gd0, d->d0, nullptr, nullptr, st))) return rc;
     // level 0 decoder: d0 = c6(u0, e0)
-    if ((rc = conv_wgrad(d, 6, d->gd0, d->u0, d->e0, W0, H0, n, st))) return rc;
     if ((rc = conv_dgrad(d, 6, d->gd0, W0, H0, n, d->gu0, d->u0, d->ge0, d->e0, st))) return rc;
     up_bwd(d->gu0, d->gd1, 64, 0);
     // level 1 decoder: d1 = c5(u1, e1)
-    if ((rc = conv_wgrad(d, 5, d->gd1, d->u1, d->e1, L[1].w, L[1].h, n, st))) return rc;
     if ((rc = conv_dgrad(d, 5, d->gd1, L[1].w, L[1].h, n, d->gu1, d->u1, d->ge1, d->e1, st))) return rc;
     up_bwd(d->gu1, d->gd2, 96, 1);
     // level 2 decoder: d2 = c4(u2, e2)
-    if ((rc = conv_wgrad(d, 4, d->gd2, d->u2, d->e2, L[2].w, L[2].h, n, st))) return rc;
     if ((rc = conv_dgrad(d, 4, d->gd2, L[2].w, L[2].h, n, d->gu2, d->u2, d->ge2, d->e2, st))) return rc;
     up_bwd(d->gu2, d->ge3, 128, 2);
     // bottleneck e3 = c3(p2)
-    if ((rc = conv_wgrad(d, 3, d->ge3, d->p2, nullptr, L[3].w, L[3].h, n, st))) return rc;
     if ((rc = conv_dgrad(d, 3, d->ge3, L[3].w, L[3].h, n, d->gp2, nullptr, nullptr, nullptr, st))) return rc;
     pool_bwd(d->gp2, d->e2, d->ge2, 96, 2);
     // encoder e2 = c2(p1)
-    if ((rc = conv_wgrad(d, 2, d->ge2, d->p1, nullptr, L[2].w, L[2].h, n, st))) return rc;
     if ((rc = conv_dgrad(d, 2, d->ge2, L[2].w, L[2].h, n, d->gp1, nullptr, nullptr, nullptr, st))) return rc;
     pool_bwd(d->gp1, d->e1, d->ge1, 64, 1);
     // encoder e1 = c1(p0)
-    if ((rc = conv_wgrad(d, 1, d->ge1, d->p0, nullptr, L[1].w, L[1].h, n, st))) return rc;
     if ((rc = conv_dgrad(d, 1, d->ge1, L[1].w, L[1].h, n, d->gp0, nullptr, nullptr, nullptr, st))) return rc;
     pool_bwd(d->gp0, d->e0, d->ge0, 32, 0);
     // encoder e0 = c0(x)
-    if ((rc = conv_wgrad(d, 0, d->ge0, x, nullptr, W0, H0, n, st))) return rc;
+    // every layer's weight gradient: the activations and their gradients are all still there
+    WgradBatch wg(d->d_err, st);
+    if ((rc = conv_wgrad(d, wg, 7, d->gy, d->d0, nullptr, W0, H0, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 6, d->gd0, d->u0, d->e0, W0, H0, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 5, d->gd1, d->u1, d->e1, L[1].w, L[1].h, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 4, d->gd2, d->u2, d->e2, L[2].w, L[2].h, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 3, d->ge3, d->p2, nullptr, L[3].w, L[3].h, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 2, d->ge2, d->p1, nullptr, L[2].w, L[2].h, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 1, d->ge1, d->p0, nullptr, L[1].w, L[1].h, n))) return rc;
+    if ((rc = conv_wgrad(d, wg, 0, d->ge0, x, nullptr, W0, H0, n))) return rc;
+    if ((rc = wg.launch())) return rc;
     LayerGrads G;
     const bf16* g[8] = {d->ge0, d->ge1, d->ge2, d->ge3, d->gd2, d->gd1, d->gd0, d->gy};
     const int level[8] = {0, 1, 2, 3, 2, 1, 0, 0};
