@@ -69,3 +69,27 @@ def test_forward_takes_any_placement(cuda):
     _abi.check(_abi.lib().rl_denoiser_forward(dn.handle, C.c_void_p(same.data_ptr()), 1, 40, 40,
                                               C.c_void_p(same.data_ptr()), None))
     assert torch.equal(same[..., :3], want[..., :3])
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 16, 16), (3, 160, 72)])
+def test_masked_gradient_columns(cuda, n, h, w):
+    """A data gradient of 32 channels into 128 columns of which 96 are kept, in
+    one tile per CTA and in several (two issuers, two accumulator sets), against
+    FP32; BF16 outputs of sums of 288 products: 2^-8 of the value and 2^-8 of
+    the largest."""
+    import torch
+    from relight_b200 import denoise as D
+    g = torch.Generator(device="cuda").manual_seed(h)
+    x = torch.randn(n, h, w, 32, device="cuda", generator=g).bfloat16()
+    wt = (torch.randn(128, 32, 3, 3, device="cuda", generator=g) * 0.1).bfloat16()
+    wp = wt.permute(2, 3, 1, 0).reshape(9, 4, 8, 128).permute(0, 1, 3, 2).contiguous()
+    m0, m1 = (torch.randn(n, h, w, c, device="cuda", generator=g).bfloat16() for c in (64, 32))
+    o0, o1 = torch.zeros_like(m0), torch.zeros_like(m1)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    D.conv3x3(x, wp, 128, out0=o0, out0_c0=0, out0_cn=64, mask0=m0, out1=o1, out1_c0=64, out1_cn=32, mask1=m1, err=err)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), wt.double(), padding=1).permute(0, 2, 3, 1)
+    for got, r in ((o0, ref[..., :64] * (m0 > 0)), (o1, ref[..., 64:96] * (m1 > 0))):
+        d = (got.double() - r).abs()
+        assert bool((d <= 2.0 ** -8 * (r.abs() + r.abs().max())).all()), float(d.max())
