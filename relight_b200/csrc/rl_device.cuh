@@ -27,6 +27,8 @@ namespace rl {
 // Triangles, 48 bytes in leaf order: t0 = v0.xyz | gid bits, t1 = e1.xyz, t2 = e2.xyz.
 struct DevScene {
     const float4* nodes;
+    const uint4* qnodes;        // the nodes in 32 bytes each (QSlab), or null
+    float qlo[3], qstep[3];     // their grid
     const float4* nodes4;       // 4-wide nodes, 128 B: lo.x hi.x lo.y hi.y lo.z hi.z (4 children each), codes, pad
     const float4* tris;
     const int4* tri_vidx;       // per global triangle id: a, b, c, mesh
@@ -330,6 +332,72 @@ __device__ __forceinline__ void slab2(float4 n0, float4 n1, float4 n2, const Sla
     const float2 az = unpack2(fma2(wz, r.bz, tz)), bz = unpack2(fma2(wz, r.az, tz));
     const float lo0 = fmax3(a0.x, a0.y, fmaxf(az.x, tnear)), hi0 = fmin3(b0.x, b0.y, fminf(bz.x, tmax));
     const float lo1 = fmax3(a1.x, a1.y, fmaxf(az.y, tnear)), hi1 = fmin3(b1.x, b1.y, fminf(bz.y, tmax));
+    h0 = lo0 <= hi0 * 1.0000003f;
+    h1 = lo1 <= hi1 * 1.0000003f;
+    e0 = lo0;
+    e1 = lo1;
+}
+
+// 32 bytes (32-byte aligned) in one load.
+__device__ __forceinline__ void ldg32(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// A node in 32 bytes: per child the x, y, z planes as lo | hi << 16 in steps of
+// a grid over the scene, and the child's code.  Lanes at different nodes cost
+// the L1 one pass each per load whatever its width, and those passes bound the
+// walks of incoherent rays, so that one load a node in place of four counts
+// there (1M closest hits 194 -> 160 us, 4M any hits 624 -> 465; two 32-byte
+// loads of the full nodes: 184 and 565).  Warps whose rays keep together are
+// bound by the instructions, of which this takes nine more: their kernels
+// keep the full nodes (terrain final gather 25.5 -> 25.8 ms with these).
+//
+// A 16-bit plane q becomes 2^23 + q by a byte permutation, and
+// t = (2^23 + q) step / d + b.  b is rounded at half a step of the grid over d
+// and at 2^-24 of the origin's distance from the grid, two or three times: the
+// planes lie two steps further out than the box (k_quantize_nodes), which
+// covers origins up to 100 scene sizes away; the padding of the full nodes'
+// planes, 1e-5 of the largest coordinate, which these have as well, ends at 50.
+struct QSlab {
+    f32x2 ax, ay, az, bx, by, bz;   // step / d and (grid origin - o) / d - 2^23 step / d, twice each
+    uint32_t sx, sy, sz;            // byte selectors of the nearer plane
+};
+__device__ __forceinline__ QSlab make_qslab(const DevScene& s, V3 o, V3 d) {
+    QSlab r;
+    auto axis = [](float o, float d, float lo, float step, f32x2& a2, f32x2& b2, uint32_t& sel) {
+        const float inv = slab_inv(d);
+        const float a = step * inv, b = __fmaf_rn(-8388608.0f, a, (lo - o) * inv);
+        a2 = pack2(a, a);
+        b2 = pack2(b, b);
+        sel = signbit(inv) ? 0x7432u : 0x7410u;
+    };
+    axis(o.x, d.x, s.qlo[0], s.qstep[0], r.ax, r.bx, r.sx);
+    axis(o.y, d.y, s.qlo[1], s.qstep[1], r.ay, r.by, r.sy);
+    axis(o.z, d.z, s.qlo[2], s.qstep[2], r.az, r.bz, r.sz);
+    return r;
+}
+__device__ __forceinline__ float qplane(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)); }
+
+// Both children of a node, as slab2: tests against [tnear, tmax], entry distances, codes.
+__device__ __forceinline__ void qvisit(const DevScene& s, int node, const QSlab& r, float tnear, float tmax, bool& h0,
+                                       bool& h1, float& e0, float& e1, int& c0, int& c1) {
+    float4 f0, f1;
+    ldg32(reinterpret_cast<const float4*>(s.qnodes + 2 * (size_t)node), f0, f1);
+    const uint32_t x0 = __float_as_uint(f0.x), y0 = __float_as_uint(f0.y), z0 = __float_as_uint(f0.z);
+    const uint32_t x1 = __float_as_uint(f1.x), y1 = __float_as_uint(f1.y), z1 = __float_as_uint(f1.z);
+    c0 = __float_as_int(f0.w);
+    c1 = __float_as_int(f1.w);
+    const uint32_t fx = r.sx ^ 0x22u, fy = r.sy ^ 0x22u, fz = r.sz ^ 0x22u;
+    const float2 nx = unpack2(fma2(pack2(qplane(x0, r.sx), qplane(x1, r.sx)), r.ax, r.bx));
+    const float2 ny = unpack2(fma2(pack2(qplane(y0, r.sy), qplane(y1, r.sy)), r.ay, r.by));
+    const float2 nz = unpack2(fma2(pack2(qplane(z0, r.sz), qplane(z1, r.sz)), r.az, r.bz));
+    const float2 gx = unpack2(fma2(pack2(qplane(x0, fx), qplane(x1, fx)), r.ax, r.bx));
+    const float2 gy = unpack2(fma2(pack2(qplane(y0, fy), qplane(y1, fy)), r.ay, r.by));
+    const float2 gz = unpack2(fma2(pack2(qplane(z0, fz), qplane(z1, fz)), r.az, r.bz));
+    const float lo0 = fmax3(nx.x, ny.x, fmaxf(nz.x, tnear)), hi0 = fmin3(gx.x, gy.x, fminf(gz.x, tmax));
+    const float lo1 = fmax3(nx.y, ny.y, fmaxf(nz.y, tnear)), hi1 = fmin3(gx.y, gy.y, fminf(gz.y, tmax));
     h0 = lo0 <= hi0 * 1.0000003f;
     h1 = lo1 <= hi1 * 1.0000003f;
     e0 = lo0;
