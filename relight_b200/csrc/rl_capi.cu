@@ -1026,6 +1026,97 @@ extern "C" int rl_map_add_mesh(rl_map* m, const rl_scene* s, int mesh, void* str
     return RL_OK;
 }
 
+namespace {
+// Pinned host memory for results: a copy into it does not wait, one into
+// pageable memory does (about 10 us each, and 4 to 6 GB/s for a large one).  A
+// call takes one block from a few that the process keeps, or pins its own when
+// they are all out (about a millisecond); a block that a failed call may still
+// have a copy in flight to is not kept.
+struct PinnedStaging {
+    static constexpr size_t kBytes = 1 << 20, kKept = 4;
+    char* p = nullptr;
+    bool settled = true;   // no copy in flight
+    int reserve() {
+        {
+            std::lock_guard<std::mutex> lk(mutex());
+            if (!kept().empty()) {
+                p = kept().back();
+                kept().pop_back();
+            }
+        }
+        if (!p) CK(cudaMallocHost((void**)&p, kBytes));
+        settled = false;
+        return RL_OK;
+    }
+    ~PinnedStaging() {
+        if (!p) return;
+        if (settled) {
+            std::lock_guard<std::mutex> lk(mutex());
+            if (kept().size() < kKept) {
+                kept().push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);   // waits for the device
+    }
+
+   private:
+    static std::mutex& mutex() {
+        static std::mutex mu;
+        return mu;
+    }
+    static std::vector<char*>& kept() {
+        static std::vector<char*>* blocks = new std::vector<char*>;   // outlives the last call at exit
+        if (blocks->capacity() < kKept) blocks->reserve(kKept);
+        return *blocks;
+    }
+};
+
+// Device to host, done when it returns.  Pageable memory is filled by this
+// thread from the two halves of a pinned block, one while the other arrives:
+// a 1024^2 RGBM image, 4 MB into a fresh array, 646 -> 460 us, most of it the
+// host's copy (1,038 -> 470 on another host; into pinned memory 123, which
+// takes the direct copy).  Halves of 256 and 128 KB: 485 and 560 us.
+constexpr size_t kStagedBytes = 32 << 10;
+
+int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    cudaPointerAttributes at;
+    PinnedStaging pin;
+    const bool staged = bytes >= kStagedBytes && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+                        at.type == cudaMemoryTypeUnregistered && pin.reserve() == RL_OK;
+    if (!staged) {
+        cudaGetLastError();
+        pin.settled = true;
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        return RL_OK;
+    }
+    constexpr size_t half = PinnedStaging::kBytes / 2;
+    const size_t parts = (bytes + half - 1) / half;
+    struct Events {
+        cudaEvent_t e[2] = {nullptr, nullptr};
+        ~Events() {
+            for (cudaEvent_t x : e)
+                if (x) cudaEventDestroy(x);
+        }
+    } ev;
+    for (cudaEvent_t& x : ev.e) CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+    for (size_t k = 0; k < parts + 1; k++) {
+        if (k < parts) {
+            CK(cudaMemcpyAsync(pin.p + k % 2 * half, (const char*)src + k * half, std::min(half, bytes - k * half),
+                               cudaMemcpyDeviceToHost, st));
+            CK(cudaEventRecord(ev.e[k % 2], st));
+        }
+        if (k > 0) {
+            CK(cudaEventSynchronize(ev.e[(k - 1) % 2]));
+            std::memcpy((char*)dst + (k - 1) * half, pin.p + (k - 1) % 2 * half, std::min(half, bytes - (k - 1) * half));
+        }
+    }
+    pin.settled = true;
+    return RL_OK;
+}
+}  // namespace
+
 // The status of a blur queued on `m`, read by the calls that wait for it.
 static int read_blur_status(const rl_map* m, cudaStream_t st, int* status) {
     *status = 0;
@@ -1042,13 +1133,20 @@ extern "C" int rl_map_download(const rl_map* m, int32_t* flags, int32_t* face, f
     if (!m) return fail(RL_INVALID_CALL, "null map");
     cudaStream_t st = S(stream);
     size_t n = (size_t)m->dev.width * m->dev.height;
-    if (flags) CK(cudaMemcpyAsync(flags, m->dev.flags, 4 * n, cudaMemcpyDeviceToHost, st));
-    if (face) CK(cudaMemcpyAsync(face, m->dev.face, 4 * n, cudaMemcpyDeviceToHost, st));
-    if (position) CK(cudaMemcpyAsync(position, m->dev.position, 12 * n, cudaMemcpyDeviceToHost, st));
-    if (normal) CK(cudaMemcpyAsync(normal, m->dev.normal, 12 * n, cudaMemcpyDeviceToHost, st));
-    if (color) CK(cudaMemcpyAsync(color, m->dev.color, 12 * n, cudaMemcpyDeviceToHost, st));
-    if (photons) CK(cudaMemcpyAsync(photons, m->dev.photons, 4 * n, cudaMemcpyDeviceToHost, st));
-    if (gathered) CK(cudaMemcpyAsync(gathered, m->dev.gathered, 12 * n, cudaMemcpyDeviceToHost, st));
+    if (flags)
+        if (int rc = copy_to_host(flags, m->dev.flags, 4 * n, st)) return rc;
+    if (face)
+        if (int rc = copy_to_host(face, m->dev.face, 4 * n, st)) return rc;
+    if (position)
+        if (int rc = copy_to_host(position, m->dev.position, 12 * n, st)) return rc;
+    if (normal)
+        if (int rc = copy_to_host(normal, m->dev.normal, 12 * n, st)) return rc;
+    if (color)
+        if (int rc = copy_to_host(color, m->dev.color, 12 * n, st)) return rc;
+    if (photons)
+        if (int rc = copy_to_host(photons, m->dev.photons, 4 * n, st)) return rc;
+    if (gathered)
+        if (int rc = copy_to_host(gathered, m->dev.gathered, 12 * n, st)) return rc;
     int blur = 0;
     if (int rc = read_blur_status(m, st, &blur)) return rc;
     CK(cudaStreamSynchronize(st));
@@ -2332,53 +2430,6 @@ __global__ void k_ff_finish(int n, const long long* row_ptr, const int2* entries
     for (long long k = lane; k < len; k += 32) vals[b + k] = __ldcg(vals + b + k) / sum;
 }
 
-namespace {
-// Pinned host memory for small results: a copy into it does not wait, one
-// into pageable memory does (about 10 us each).  A call takes one block from a
-// few that the process keeps, or pins its own when they are all out (about a
-// millisecond); a block that a failed call may still have a copy in flight to
-// is not kept.
-struct PinnedStaging {
-    static constexpr size_t kBytes = 1 << 20, kKept = 4;
-    char* p = nullptr;
-    bool settled = true;   // no copy in flight
-    int reserve() {
-        {
-            std::lock_guard<std::mutex> lk(mutex());
-            if (!kept().empty()) {
-                p = kept().back();
-                kept().pop_back();
-            }
-        }
-        if (!p) CK(cudaMallocHost((void**)&p, kBytes));
-        settled = false;
-        return RL_OK;
-    }
-    ~PinnedStaging() {
-        if (!p) return;
-        if (settled) {
-            std::lock_guard<std::mutex> lk(mutex());
-            if (kept().size() < kKept) {
-                kept().push_back(p);
-                return;
-            }
-        }
-        cudaFreeHost(p);   // waits for the device
-    }
-
-   private:
-    static std::mutex& mutex() {
-        static std::mutex mu;
-        return mu;
-    }
-    static std::vector<char*>& kept() {
-        static std::vector<char*>* blocks = new std::vector<char*>;   // outlives the last call at exit
-        if (blocks->capacity() < kKept) blocks->reserve(kKept);
-        return *blocks;
-    }
-};
-}  // namespace
-
 extern "C" int rl_ff_pairwise(const rl_scene* s, int n, const float* d_pos, const float* d_nrm, float threshold,
                               int64_t* row_ptr, int32_t* cols, float* vals, int64_t capacity, int64_t* nnz,
                               void* stream) {
@@ -3329,7 +3380,7 @@ extern "C" int rl_map_encode(const rl_map* m, int format, uint8_t* out, void* st
     long long bytes = encoded_bytes(m, format), n = (long long)m->dev.width * m->dev.height;
     int blur = 0;
     if (format == 0) {
-        CK(cudaMemcpyAsync(out, m->dev.color, bytes, cudaMemcpyDeviceToHost, st));
+        if (int rc = copy_to_host(out, m->dev.color, bytes, st)) return rc;
         if (int rc = read_blur_status(m, st, &blur)) return rc;
         CK(cudaStreamSynchronize(st));
         return check_blur_status(m, blur);
@@ -3342,10 +3393,10 @@ extern "C" int rl_map_encode(const rl_map* m, int format, uint8_t* out, void* st
         k_encode<<<grid_for(n, 256), 256, 0, st>>>(m->dev, format, d);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) rc = copy_to_host(out, d, bytes, st);
     cudaFreeAsync(d, st);
-    if (e == cudaSuccess) rc = read_blur_status(m, st, &blur);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && !rc) rc = read_blur_status(m, st, &blur);
+    if (e == cudaSuccess && !rc) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = fail(RL_CUDA_ERROR, "rl_map_encode: %s", cudaGetErrorString(e));
     return rc ? rc : check_blur_status(m, blur);
 }
