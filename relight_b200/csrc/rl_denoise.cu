@@ -43,6 +43,9 @@ const rl::DevScene* rl_internal_scene(const rl_scene* s);
 namespace {
 
 using bf16 = __nv_bfloat16;
+using rl::f32x2;
+using rl::pack2;
+using rl::unpack2;
 
 int dn_fail(int code, const char* fmt, ...) {
     char buf[512];
@@ -213,18 +216,27 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // Roles (one CTA per SM walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...):
 //   warp 0    tensor memory; the halo loads (HS-stage ring);
 //   warp 1    the weight copies (nine bulk copies once, or one per unit);
-//   warps 2-5 the epilogue (warp w owns TMEM lanes 32 (w % 4) .. +31), which
-//             drains accumulator set i % nbuf while the issuers fill the others;
-//   warps 6-9 the MMA issuers (lane 0 of each; warp 6 + k is issuer k);
-//   warps 10-13 a second epilogue group when there are two or more
-//             accumulator sets: groups 0 and 1 take the even and odd tiles.
+//   warps 2-5 the MMA issuers (lane 0 of each; warp 2 + k is issuer k);
+//   warps 6-21 the epilogue, four groups of four warps (warp w owns TMEM lanes
+//             32 (w % 4) .. +31): they drain accumulator set i % nbuf while the
+//             issuers fill the others.  With four sets each group takes every
+//             fourth tile, with two sets two groups share each tile's columns,
+//             with one all four do.
+// The epilogue bounds most layers (about 10 cycles an instruction for the few
+// warps that a scheduler has of it): with two groups, sums one by one and the
+// bias read from global memory for each pixel, the eight convolutions of a
+// 1024^2 map took 471 us, 423 so (16 -> 32 channels 68 -> 52, 64 -> 96 37 -> 22).
+// What is left: 160 -> 64 channels (84 us) and 224 -> 96 (56) stream their
+// weights through the L2 for every tile; tiles of two halves, which halve that,
+// leave no room for a second halo stage and came out the same.
 
 constexpr int kTileW = 16, kTileH = 8;    // the weight gradient's pixel tile: 128 pixels
 constexpr uint32_t kABytes = 128 * 128;   // 128 pixels x 64 channels x 2 bytes
 constexpr int kHTileH = 16;               // the convolution's tile: 16 rows of 8 pixels per half
 constexpr int kHaloH = kHTileH + 2;
 constexpr int kMaxIssuers = 4;
-constexpr int kConvThreads = (10 + kMaxIssuers) * 32;
+constexpr int kEpiGroups = 4, kEpiWarp0 = 2 + kMaxIssuers;
+constexpr int kConvThreads = (kEpiWarp0 + 4 * kEpiGroups) * 32;
 
 struct ConvArgs {
     int W, H;              // spatial size (input = output)
@@ -311,26 +323,40 @@ __device__ __forceinline__ void tmem_regs_ready(uint32_t (&r)[16]) {
                    "+r"(r[15]));
 }
 
-// The first chunk of 16 columns from c on that an output segment takes
-// (ncols: none).
-__device__ __forceinline__ int conv_next_chunk(const ConvArgs& a, int c) {
-    for (; c < a.ncols; c += 16)
-        for (int o = 0; o < a.nout; o++)
-            if (c >= a.out_c0[o] && c < a.out_c0[o] + a.out_cn[o]) return c;
-    return c;
+// Two additions in one instruction.
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
-// One 16-column chunk of an output row: the summed accumulator values x[16]
-// of columns [c, c + 16) -> bias, activation (in place), mask -> BF16 stores
-// into the output segments that hold those columns.
-__device__ __forceinline__ void conv_store_chunk(const ConvArgs& a, int c, float (&x)[16], long long pix) {
+// One 16-column chunk of an output row: the summed accumulator values
+// of columns [c, c + 16) -> bias, activation.
+__device__ __forceinline__ void conv_activate(const ConvArgs& a, const float* bias, int c, const f32x2 (&v)[8],
+                                              float (&x)[16]) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        float t = x[i];
-        if (a.bias) t += a.bias[c + i];
-        if (a.relu && !(t > 0.0f)) t *= a.slope;
-        x[i] = t;
+    for (int i = 0; i < 8; i += 2) {
+        f32x2 t0 = v[i], t1 = v[i + 1];
+        if (a.bias) {
+            const float4 b = *reinterpret_cast<const float4*>(bias + c + 2 * i);
+            t0 = add2(t0, pack2(b.x, b.y));
+            t1 = add2(t1, pack2(b.z, b.w));
+        }
+        const float2 f0 = unpack2(t0), f1 = unpack2(t1);
+        x[2 * i] = f0.x;
+        x[2 * i + 1] = f0.y;
+        x[2 * i + 2] = f1.x;
+        x[2 * i + 3] = f1.y;
     }
+    if (a.relu) {
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            if (!(x[i] > 0.0f)) x[i] *= a.slope;
+    }
+}
+
+// ... -> mask -> BF16 stores into the output segments that hold those columns.
+__device__ __forceinline__ void conv_store_chunk(const ConvArgs& a, int c, const float (&x)[16], long long pix) {
     for (int o = 0; o < a.nout; o++) {
         if (c < a.out_c0[o] || c >= a.out_c0[o] + a.out_cn[o]) continue;
         const long long off = pix * a.out_cs[o] + (c - a.out_c0[o]);
@@ -364,21 +390,21 @@ __device__ __forceinline__ void conv_store_chunk(const ConvArgs& a, int c, float
 // (taddr = lane, column 0 of the tile's first partial; partial k starts k x
 // pstride columns further), summed; two partials per load round keep the
 // registers in use at 32.
-__device__ __forceinline__ void conv_sum_chunk(const ConvArgs& a, uint32_t taddr, int col, float (&x)[16]) {
+__device__ __forceinline__ void conv_sum_chunk(const ConvArgs& a, uint32_t taddr, int col, f32x2 (&x)[8]) {
 #pragma unroll
     for (int k0 = 0; k0 < kMaxIssuers; k0 += 2) {
-        if (k0 >= a.issuers) break;
+        if (k0 >= a.issuers) break;   // two or four
         uint32_t r0[16], r1[16];
         tmem_ld16_async(taddr + (uint32_t)(k0 * a.pstride + col), r0);
-        if (k0 + 1 < a.issuers) tmem_ld16_async(taddr + (uint32_t)((k0 + 1) * a.pstride + col), r1);
+        tmem_ld16_async(taddr + (uint32_t)((k0 + 1) * a.pstride + col), r1);
         tmem_wait_ld();
         tmem_regs_ready(r0);
-        if (k0 + 1 < a.issuers) tmem_regs_ready(r1);
+        tmem_regs_ready(r1);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            float t = __uint_as_float(r0[i]);
-            if (k0 + 1 < a.issuers) t += __uint_as_float(r1[i]);
-            x[i] = k0 == 0 ? t : x[i] + t;
+        for (int i = 0; i < 8; i++) {
+            const f32x2 t = add2(pack2(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1])),
+                                 pack2(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1])));
+            x[i] = k0 == 0 ? t : add2(x[i], t);
         }
     }
 }
@@ -395,70 +421,75 @@ __device__ __forceinline__ TileXY tile_xy(int tile, int tiles_x, int tiles_y, in
 }
 
 // Epilogue of one tile for this thread's TMEM lane (pixel row % 8, row / 8 of
-// each 8-pixel half; half h's accumulator starts h x tmem_cols columns on),
-// then the accumulator set's release (`drained`).  When the tile has at most
-// 64 columns in all (halves x ncols) and no mask, the finished BF16 values
-// are held in registers and the set is released before the global stores, so
-// the release (which orders this thread's earlier memory operations) does not
-// wait for them; otherwise the row is stored chunk by chunk and released
-// after.
+// each 8-pixel half; half h's accumulator starts h x tmem_cols columns on):
+// the 16-column chunks part, part + parts, ... of the tile's halves x ncols,
+// then the accumulator set's release (`drained`).  When that is at most two
+// chunks and there is no mask, the finished BF16 values are held in registers
+// and the set is released before the global stores, so the release (which
+// orders this thread's earlier memory operations) does not wait for them;
+// otherwise each chunk is stored in its turn and the set released after.
 template <int kHalves>
-__device__ __forceinline__ void conv_epilogue_tile(const ConvArgs& a, uint32_t taddr, const TileXY& tx, int row,
-                                                   bool ready, uint64_t* drained) {
-    const int cpc = a.ncols / 16;  // 16-column chunks per half
+__device__ __forceinline__ void conv_epilogue_tile(const ConvArgs& a, const float* bias, uint32_t taddr,
+                                                   const TileXY& tx, int row, bool ready, uint64_t* drained, int part,
+                                                   int parts) {
+    const int cpc = a.ncols / 16;  // chunks per half
     auto pixel = [&](int h, long long& pix) {
         const int px = tx.x0 + 8 * h + (row & 7), py = tx.y0 + (row >> 3);
         pix = ((long long)tx.img * a.H + py) * a.W + px;
         return ready && px < a.W && py < a.H;
     };
-    if (kHalves * a.ncols <= 64 && !a.mask[0] && !a.mask[1]) {
-        // finished BF16 values, 16 bytes per 8 columns
-        uint4 q[4][2];
+    auto takes = [&](int o, int c) { return o < a.nout && c >= a.out_c0[o] && c < a.out_c0[o] + a.out_cn[o]; };
+    if (kHalves * cpc <= 2 * parts && !a.mask[0] && !a.mask[1]) {
+        uint4 q[2][2];
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int k = 0; k < 2; k++) {
+            const int j = part + k * parts;
             if (j < kHalves * cpc) {
-                const int h = j / cpc, c = 16 * (j - h * cpc);
+                const int h = kHalves == 2 && j >= cpc, c = 16 * (j - h * cpc);
+                f32x2 v[8];
                 float x[16];
-                conv_sum_chunk(a, taddr + (uint32_t)(h * a.tmem_cols), c, x);
-                __nv_bfloat162* p0 = reinterpret_cast<__nv_bfloat162*>(&q[j][0]);
-                __nv_bfloat162* p1 = reinterpret_cast<__nv_bfloat162*>(&q[j][1]);
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    float t = x[i];
-                    if (a.bias) t += a.bias[c + i];
-                    if (a.relu && !(t > 0.0f)) t *= a.slope;
-                    x[i] = t;
-                }
+                conv_sum_chunk(a, taddr + (uint32_t)(h * a.tmem_cols), c, v);
+                conv_activate(a, bias, c, v, x);
+                __nv_bfloat162* p0 = reinterpret_cast<__nv_bfloat162*>(&q[k][0]);
+                __nv_bfloat162* p1 = reinterpret_cast<__nv_bfloat162*>(&q[k][1]);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     p0[i] = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
                     p1[i] = __floats2bfloat162_rn(x[8 + 2 * i], x[8 + 2 * i + 1]);
                 }
             }
+        }
         tc_fence_before();
         mbar_arrive(drained);
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int k = 0; k < 2; k++) {
+            const int j = part + k * parts;
             if (j < kHalves * cpc) {
-                const int h = j / cpc, c = 16 * (j - h * cpc);
+                const int h = kHalves == 2 && j >= cpc, c = 16 * (j - h * cpc);
                 long long pix;
                 if (!pixel(h, pix)) continue;
-                for (int o = 0; o < a.nout; o++) {
-                    if (c < a.out_c0[o] || c >= a.out_c0[o] + a.out_cn[o]) continue;
+#pragma unroll
+                for (int o = 0; o < 2; o++) {
+                    if (!takes(o, c)) continue;
                     uint4* dst = reinterpret_cast<uint4*>(a.out[o] + pix * a.out_cs[o] + (c - a.out_c0[o]));
-                    dst[0] = q[j][0];
-                    dst[1] = q[j][1];
+                    dst[0] = q[k][0];
+                    dst[1] = q[k][1];
                 }
             }
+        }
         return;
     }
-    for (int h = 0; h < kHalves; h++) {
+    for (int j = part; j < kHalves * cpc; j += parts) {
+        const int h = kHalves == 2 && j >= cpc, c = 16 * (j - h * cpc);
+        if (!takes(0, c) && !takes(1, c)) continue;   // padding between two segments
         long long pix;
         const bool inb = pixel(h, pix);
-        for (int c = conv_next_chunk(a, 0); c < a.ncols; c = conv_next_chunk(a, c + 16)) {
-            float x[16];
-            conv_sum_chunk(a, taddr + (uint32_t)(h * a.tmem_cols), c, x);
-            if (inb) conv_store_chunk(a, c, x, pix);
+        f32x2 v[8];
+        float x[16];
+        conv_sum_chunk(a, taddr + (uint32_t)(h * a.tmem_cols), c, v);
+        if (inb) {
+            conv_activate(a, bias, c, v, x);
+            conv_store_chunk(a, c, x, pix);
         }
     }
     tc_fence_before();
@@ -479,8 +510,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     uint64_t* bfull = hempty + HS;
     uint64_t* bempty = bfull + BS;
     uint64_t* accf = bempty + BS;  // accumulator set k ready for the epilogue (one commit per issuer)
-    uint64_t* acce = accf + 4;     // accumulator set k drained (128 epilogue threads)
+    uint64_t* acce = accf + 4;     // accumulator set k drained (by the groups that share a tile)
     uint32_t* tmem_slot = (uint32_t*)(acce + 4);
+    float* s_bias = (float*)(tmem_slot + 4);  // [256], 16-byte aligned
     const uint32_t tmem_total = 512;  // the issuers' column ranges, 512 / issuers apart
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_trigger();
@@ -495,7 +527,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         }
         for (int k = 0; k < 4; k++) {
             mbar_init(accf + k, (uint32_t)NI);
-            mbar_init(acce + k, 128);
+            mbar_init(acce + k, (uint32_t)(kEpiGroups / NB) * 128);
         }
         fence_barrier_init();
     }
@@ -561,25 +593,28 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                     mbar_wait(bfull + k % BS, (uint32_t)((k / BS) & 1), a.err, 64);
             }
         }
-    } else if (warp <= 5 || (warp >= 6 + kMaxIssuers && NB >= 2)) {
-        // epilogue group 0 (warps 2-5) takes every tile when there is one
-        // accumulator set; with two, group 1 (warps 10-13) takes the odd tiles
-        const int group = warp <= 5 ? 0 : 1, ngroup = NB >= 2 ? 2 : 1;
+    } else if (warp >= kEpiWarp0) {
+        const int e = threadIdx.x - kEpiWarp0 * 32;
+        if (a.bias)
+            for (int c = e; c < a.ncols; c += kEpiGroups * 128) s_bias[c] = a.bias[c];
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiGroups * 128) : "memory");
+        const int group = e >> 7, turns = NB, parts = kEpiGroups / turns;
+        const int turn = group % turns, part = group / turns;
         const uint32_t quarter = (uint32_t)(warp & 3);
         const int row = (int)quarter * 32 + lane;
-        int i = group;
-        for (int tile = blockIdx.x + group * gridDim.x; tile < ntiles; tile += ngroup * gridDim.x, i += ngroup) {
+        int i = turn;
+        for (int tile = blockIdx.x + turn * gridDim.x; tile < ntiles; tile += turns * gridDim.x, i += turns) {
             const int buf = i % NB;
             const bool ready = mbar_wait(accf + buf, (uint32_t)((i / NB) & 1), a.err, 4);
             tc_fence_after();
             const TileXY tx = tile_xy(tile, tiles_x, tiles_y, 8 * kHalves);
-            conv_epilogue_tile<kHalves>(a, tmem + (quarter * 32u << 16) + (uint32_t)(buf * kHalves * a.tmem_cols), tx,
-                                        row, ready, acce + buf);
+            conv_epilogue_tile<kHalves>(a, s_bias, tmem + (quarter * 32u << 16) + (uint32_t)(buf * kHalves * a.tmem_cols),
+                                        tx, row, ready, acce + buf, part, parts);
             if (!ready) break;
         }
-    } else if (warp >= 6 && warp - 6 < NI) {
+    } else if (warp - 2 < NI) {
         if (lane == 0) {
-            const int w = warp - 6;
+            const int w = warp - 2;
             const uint32_t idesc = idesc_bf16(a.ncols, false, false);
             const uint32_t lbo_b = (uint32_t)a.ncols * 16;
             // descriptor halves (umma_lh): A rows of 8 pixels halo_w x 16 bytes
@@ -942,7 +977,7 @@ extern "C" int rl_dn_conv3x3(const void* in0, int c0, const void* in1, int c1, i
     // sets (measured at 1024^2: 16 -> 32 channels 69 -> 63 us, 32 -> 3
     // channels 70 -> 54 us; with more input channels, or with one accumulator
     // set, the wider tile was slower); otherwise 16 x 8.
-    const long long budget = 225 * 1024;
+    const long long budget = 225 * 1024 - 512;  // beside the barriers and the bias
     const long long tap = a.tap_bytes, step = (long long)ncols * 32;
     const int nk16 = a.nkc_total / 2;
     auto plane_of = [](int halo_w) { return (uint32_t)((halo_w * kHaloH * 16 + 127) / 128 * 128); };
@@ -1000,7 +1035,7 @@ extern "C" int rl_dn_conv3x3(const void* in0, int c0, const void* in1, int c1, i
     // one CTA per SM: at least 116 KB of shared memory each, so two CTAs
     // never contend for tensor memory
     const long long need = (a.resident ? 9 * tap : (long long)a.bslots * a.unit_bytes) + (long long)a.hstages * halo +
-                           (2LL * a.hstages + 2LL * a.bslots + 8) * 8 + 16 + 1024;
+                           (2LL * a.hstages + 2LL * a.bslots + 8) * 8 + 16 + 256 * 4 + 1024;
     const int smem = (int)std::max<long long>(need, 116 * 1024);
     static int sms = 0;
     static std::once_flag attr;
