@@ -48,9 +48,8 @@ UNIT = "texels/s"
 WORKLOAD = "terrain 256^2 verts + 2000 boxes (154,050 tris), 1M photons x3 bounces, gather r7, FG 256 spp, 1024^2"
 L2_BYTES = 126 << 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one full-size
-# k_indirect launch in one ncu capture, and the build it was captured on.
-FG_DRAM_TRAFFIC = {"bytes": 85_620_000, "captured_on": "k_indirect<2> with per-triangle shading records and "
-                   "three-input min/max slab tests (79.87 MB read + 5.75 MB written, 41.33 ms launch under ncu)"}
+# final-gather launch in one ncu capture, and the build it was captured on.
+FG_DRAM_TRAFFIC = {"bytes": 86_950_000, "captured_on": "k_indirect_patch (79.62 MB read + 7.33 MB written)"}
 
 
 def load_peaks():
@@ -153,7 +152,7 @@ def gpu_arm(args, rank, world, local_rank):
     amb = (C.c_float * 3)(*[float(x) for x in st.ambient_color])
     valid = lmap.valid_count()
     rays_per_step = valid * st.final_gather_samples
-    launches_per_step = 3  # k_photons, k_gather, k_indirect
+    launches_per_step = 3  # k_photons, k_gather_tile, k_indirect_patch
 
     ev = lambda: torch.cuda.Event(enable_timing=True)
 
@@ -170,7 +169,7 @@ def gpu_arm(args, rank, world, local_rank):
     if knn:
         from relight_b200.device import PhotonRecords
         records = PhotonRecords(8 << 20)
-        # k_knn_bounds, k_knn_grid, k_knn_keys, radix sort (counted as one), k_knn_scatter, k_knn_start, k_knn_query
+        # k_knn_bounds, k_knn_grid, k_knn_keys, k_knn_totals, k_knn_start, k_knn_scatter, k_knn_query
         launches_per_step += 7
 
     def step(seed, fg_events=None, knn_events=None, lmap_ready=None):
@@ -323,7 +322,7 @@ def gpu_arm(args, rank, world, local_rank):
         **({"knn_ms": sum(knn_ms) / len(knn_ms)} if knn else {}),
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": e2e_total / args.steps},
-        "roofline": {"kernel": "k_indirect (final gather)", "bound": bound, "achieved": achieved,
+        "roofline": {"kernel": "k_indirect_patch (final gather)", "bound": bound, "achieved": achieved,
                      "peak": l2.value if bound == "l2" else peak, "unit": "GB/s",
                      "frac": achieved / (l2.value if bound == "l2" else peak),
                      "peak_source": ("L2 read bandwidth measured in this run by the library's probe "
@@ -925,7 +924,7 @@ def room_arm(args):
         "ao_grays_per_s": ao_rays / (ao_avg_ms / 1e3) / 1e9,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": sum(e2e_ms) / args.steps},
-        "roofline": {"kernel": "k_ao (AO 64 spp)", "bound": "l1", "achieved": achieved, "peak": l1.value,
+        "roofline": {"kernel": "k_ao_patch (AO 64 spp)", "bound": "l1", "achieved": achieved, "peak": l1.value,
                      "unit": "GB/s", "frac": achieved / l1.value,
                      "peak_source": ("L1 read bandwidth measured in this run by the library's probe "
                                      "(rl_measure_l1_read_bandwidth: 64 KiB per block re-read 2,000 times)"),
@@ -1152,7 +1151,7 @@ def radiosity_arm(args):
         "e2e": {"value": e2e_value, "unit": "Grays/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": sum(e2e_ms) / steps,
                 "note": "patch positions and normals, E and rho up from pinned memory; form factors and solve; B down"},
-        "roofline": {"kernel": "k_jacobi4_smem (50 iterations; the iterate staged in shared memory per block)", "bound": jac_bound, "achieved": achieved,
+        "roofline": {"kernel": "k_jacobi4_quads_smem (50 iterations; the iterate staged in shared memory per block)", "bound": jac_bound, "achieved": achieved,
                      "peak": l2.value if jac_bound == "l2" else peak, "unit": "GB/s",
                      "frac": achieved / (l2.value if jac_bound == "l2" else peak),
                      "peak_source": ("L2 read bandwidth measured in this run by the library's probe "
@@ -1161,9 +1160,9 @@ def radiosity_arm(args):
                      "working_set_bytes": jac_set, "traffic": None,
                      "algorithmic_bytes": jac_bytes, "bytes_per_iteration": "8 B per nonzero + 44 B per row",
                      "hbm": {"peak": peak, "source": peak_kind, "frac": achieved / peak}},
-        # k_ff_hemi_rays / _rle / _compact, k_pack4, k_jacobi4 per iteration, k_unpack4
+        # k_ff_hemi_rays / _rle / _compact, k_ff_rows, k_pack4, k_jacobi4_quads_smem per iteration, k_unpack4
         "pairwise_form_factors": pairwise,
-        "gpu_launches": (5 + iters) * steps,
+        "gpu_launches": (6 + iters) * steps,
         "clocks": clocks.summary(),
     }
     return result

@@ -375,7 +375,7 @@ size_t blur_smem(int W) { return 3 * kBandsPerCta * (size_t)blur_part(W); }
 
 }  // namespace
 
-// Maps that the cluster covers: the inboxes fit in shared memory (up to 7,500 columns) and the bands in a grid.
+// Maps that the cluster covers: rings and inboxes fit in shared memory (up to 5,800 columns) and the bands in a grid.
 bool rl_internal_blur_fits(int W, int H) {
     return W <= (1 << 20) && blur_smem(W) <= kMaxSmem && (H - 2 + kRows - 1) / kRows <= 65535;
 }
