@@ -209,6 +209,25 @@ int rl_internal_tune(int param) { return g_tune[param]; }
 
 // ------------------------------------------------------------- scene
 
+// The stack that a walk of the 4-wide nodes can need: a node's other children
+// beside what the deepest of them needs.  Children follow their parent.
+static int stack_need4(const std::vector<float>& nodes4) {
+    const size_t n = nodes4.size() / 32;
+    std::vector<int> need(n, 0);
+    for (size_t i = n; i-- > 0;) {
+        int kids = 0, deepest = 0;
+        for (int k = 0; k < 4; k++) {
+            int code;
+            std::memcpy(&code, &nodes4[32 * i + 24 + k], 4);
+            if (code == kNodeDone) continue;   // empty slot
+            kids++;
+            if (code >= 0) deepest = std::max(deepest, need[(size_t)code]);
+        }
+        need[i] = std::max(kids - 1, 0) + deepest;
+    }
+    return n ? need[0] : 0;
+}
+
 // The nodes on a 16-bit grid (QSlab), each plane two steps further out, and the
 // areas of the child boxes before and after: the number of nodes that a random
 // ray visits goes with their sum.
@@ -307,6 +326,7 @@ extern "C" int rl_scene_create(const rl_scene_desc* d, int builder, void* stream
         delete s;
         return fail(RL_INVALID_CALL, "BVH build: %s", err);
     }
+    const int stack4 = stack_need4(b.nodes4);
     s->nnodes = (int64_t)(b.nodes.size() / 16);
     s->leaves = b.leaves;
     s->depth = b.depth;
@@ -435,6 +455,7 @@ extern "C" int rl_scene_create(const rl_scene_desc* d, int builder, void* stream
     DevScene& v = s->dev;
     v.nodes = nodes; v.nodes4 = nodes4; v.tris = tris; v.tri_vidx = dvidx; v.shade = dshade;
     v.nodes8 = nodes8; v.tris8 = tris8;
+    v.wide = nodes4 && stack4 <= kStackSize;
     v.pos = pos; v.nrm = nrm; v.uv0 = uv0; v.uv1 = uv1; v.vmat = dvmat;
     v.mesh_first_tri = first; v.mesh_photonmap = dpmap;
     v.mat_rgb = mat_rgb; v.mat_tex = dmat_tex; v.tex_dims = tex_dims; v.tex_offset = tex_off; v.tex_pixels = tex_px;
@@ -475,12 +496,21 @@ extern "C" int rl_scene_status(rl_scene* s, int clear, int32_t* flags, void* str
 
 // ------------------------------------------------------------- tracing
 
+// Up to one ray for each lane of the resident warps a launch is bound by the
+// latency of one walk: a ray a thread, over the 4-wide nodes where the scene
+// has them (10,000 rays 41 -> 34 us, 75,000 49 -> 40, 150,000 60 -> 56;
+// k_intersect_rays 49, 54 and 57).  Beyond, rl_intersect_rays takes
+// k_intersect_rays: 400,000 rays 92 us against 96 with a thread each over the
+// binary nodes, 1M 160 against 194.
+constexpr long long kFewRays = 148 * 32 * 32;
+
+template <bool kWide>
 __global__ void k_trace_segments(DevScene s, long long n, const float* seg, int flags, int* hit, float* tuv,
                                  int* mesh_face, float* point, float* normal, float* rgba, float* uv, int* status) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     SegHit r;
-    trace_segment(s, ld3(seg + 6 * i), ld3(seg + 6 * i + 3), flags, r, status);
+    trace_segment<kWide>(s, ld3(seg + 6 * i), ld3(seg + 6 * i + 3), flags, r, status);
     hit[i] = r.hit ? 1 : 0;
     if (tuv) { tuv[3 * i] = r.hit ? r.t : 0.f; tuv[3 * i + 1] = r.hit ? r.u : 0.f; tuv[3 * i + 2] = r.hit ? r.v : 0.f; }
     if (mesh_face) { mesh_face[2 * i] = r.hit ? r.mesh : -1; mesh_face[2 * i + 1] = r.hit ? r.face : -1; }
@@ -501,9 +531,9 @@ extern "C" int rl_trace_segments(const rl_scene* s, int64_t n, const float* d_se
                                  float* d_rgba, float* d_uv, void* stream) {
     if (!s || (n > 0 && (!d_seg || !d_hit))) return fail(RL_INVALID_CALL, "rl_trace_segments: null argument");
     if (n <= 0) return RL_OK;
-    k_trace_segments<<<blocks_for(n, 128), 128, 0, S(stream)>>>(s->dev, n, d_seg, flags, d_hit, d_t_uv,
-                                                                d_mesh_face, d_point, d_normal, d_rgba, d_uv,
-                                                                s->d_status);
+    (s->dev.wide && n <= kFewRays ? k_trace_segments<true> : k_trace_segments<false>)
+        <<<blocks_for(n, 128), 128, 0, S(stream)>>>(s->dev, n, d_seg, flags, d_hit, d_t_uv, d_mesh_face, d_point,
+                                                    d_normal, d_rgba, d_uv, s->d_status);
     CK_LAUNCH("k_trace_segments");
     return RL_OK;
 }
@@ -513,8 +543,9 @@ extern "C" int rl_trace_segments(const rl_scene* s, int64_t n, const float* d_se
 // on the open interval (tnear, tfar) of org + t dir, ties to the smaller
 // (geomID, primID).
 //
-// One ray a thread over the full nodes, for calls of at most kFewRays: there the
-// time is one walk's latency, and lanes that wait for each other add to it.
+// One ray a thread, for calls of at most kFewRays: lanes that wait for each other
+// would add to the latency of a walk.
+template <bool kWide>
 __global__ void k_intersect_few(DevScene s, long long n, const float4* rays, int any_hit, int* geom_prim,
                                  float* tuv, int* status) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -522,8 +553,11 @@ __global__ void k_intersect_few(DevScene s, long long n, const float4* rays, int
     const float4 a = rays[2 * i], b = rays[2 * i + 1];
     const V3 o = mk3(a.x, a.y, a.z), d = mk3(b.x, b.y, b.z);
     RayHit h;
-    const bool hit = any_hit ? traverse<true>(s, o, d, a.w, b.w, h, status)
-                             : traverse<false>(s, o, d, a.w, b.w, h, status);
+    bool hit;
+    if constexpr (kWide)
+        hit = any_hit ? traverse4<true>(s, o, d, a.w, b.w, h) : traverse4<false>(s, o, d, a.w, b.w, h);
+    else
+        hit = any_hit ? traverse<true>(s, o, d, a.w, b.w, h, status) : traverse<false>(s, o, d, a.w, b.w, h, status);
     int mesh = -1, prim = -1;
     if (hit) {
         mesh = __ldg(s.tri_vidx + h.gid).w;
@@ -658,11 +692,6 @@ __global__ void __launch_bounds__(kRayThreads) k_intersect_rays(DevScene s, long
     }
 }
 
-// Up to one ray for each lane of the resident warps.  k_intersect_few against
-// k_intersect_rays: 10,000 rays 41 and 49 us, 75,000 50 and 54, 150,000 59 and
-// 57, 400,000 96 and 92, 1M 194 and 160.
-constexpr long long kFewRays = 148 * 32 * 32;
-
 extern "C" int rl_intersect_rays(const rl_scene* s, int64_t n, const float* d_rays, int any_hit, int32_t* d_geom_prim,
                                  float* d_t_uv, void* stream) {
     if (!s || n < 0 || (n > 0 && (!d_rays || !d_geom_prim)))
@@ -671,7 +700,8 @@ extern "C" int rl_intersect_rays(const rl_scene* s, int64_t n, const float* d_ra
     if (n == 0) return RL_OK;
     const float4* rays = reinterpret_cast<const float4*>(d_rays);
     if (n <= kFewRays) {
-        k_intersect_few<<<blocks_for(n, 128), 128, 0, S(stream)>>>(s->dev, n, rays, any_hit, d_geom_prim, d_t_uv, s->d_status);
+        (s->dev.wide ? k_intersect_few<true> : k_intersect_few<false>)<<<blocks_for(n, 128), 128, 0, S(stream)>>>(
+            s->dev, n, rays, any_hit, d_geom_prim, d_t_uv, s->d_status);
         CK_LAUNCH("k_intersect_few");
         return RL_OK;
     }

@@ -29,6 +29,7 @@ struct DevScene {
     const float4* nodes;
     const uint4* qnodes;        // the nodes in 32 bytes each (QSlab), or null
     float qlo[3], qstep[3];     // their grid
+    int wide;                   // the 4-wide nodes are there and traverse4's stack holds any walk of them
     const float4* nodes4;       // 4-wide nodes, 128 B: lo.x hi.x lo.y hi.y lo.z hi.z (4 children each), codes, pad
     const float4* tris;
     const int4* tri_vidx;       // per global triangle id: a, b, c, mesh
@@ -901,6 +902,69 @@ __device__ __forceinline__ void ray_loop4(const DevScene& s, Gen& g, int refill,
     }
 }
 
+// traverse() over the 4-wide nodes: half the dependent steps for about the
+// same loads and more tests, for launches too small to hide the latency of a
+// step (10,000 rays 41 -> 34 us; a million rays, and photons with their long
+// paths, take no less).  The caller has checked that no walk can overflow the
+// stack (DevScene::wide).
+template <bool kAny>
+__device__ __forceinline__ bool traverse4(const DevScene& s, V3 o, V3 d, float tnear, float tfar, RayHit& hit) {
+    hit.gid = -1;
+    if (s.ntris == 0) return false;
+    const V3 idir = mk3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+    const V3 ood = mk3(o.x * idir.x, o.y * idir.y, o.z * idir.z);
+    int stack[kStackSize];
+    int sp = 0, node = 0;
+    float best = tfar;
+    int best_gid = 0x7fffffff;
+    for (;;) {
+        while (node >= 0) {
+            const float4* np = s.nodes4 + 8 * (size_t)node;
+            float4 lx, hx, ly, hy, lz, hz;
+            ldg32(np, lx, hx);
+            ldg32(np + 2, ly, hy);
+            ldg32(np + 4, lz, hz);
+            const int4 cc = __ldg(reinterpret_cast<const int4*>(np + 6));
+            float k0 = child_entry(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, idir, ood, tnear, best, cc.x);
+            float k1 = child_entry(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, idir, ood, tnear, best, cc.y);
+            float k2 = child_entry(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, idir, ood, tnear, best, cc.z);
+            float k3 = child_entry(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, idir, ood, tnear, best, cc.w);
+            int c0 = cc.x, c1 = cc.y, c2 = cc.z, c3 = cc.w;
+            cswap(k0, c0, k1, c1);
+            cswap(k2, c2, k3, c3);
+            cswap(k0, c0, k2, c2);
+            cswap(k1, c1, k3, c3);
+            cswap(k1, c1, k2, c2);
+            if (k3 < kMissKey) stack[sp++] = c3;
+            if (k2 < kMissKey) stack[sp++] = c2;
+            if (k1 < kMissKey) stack[sp++] = c1;
+            if (k0 < kMissKey) {
+                node = c0;
+            } else {
+                if (sp == 0) return hit.gid >= 0;
+                node = stack[--sp];
+            }
+        }
+        const int code = ~node;
+        const int first = code >> 3, count = (code & 7) + 1;
+        for (int i = first; i < first + count; i++) {
+            const float4* tp = s.tris + 3 * (size_t)i;
+            const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
+            float t, u, v;
+            if (tri_test(t0, t1, t2, o, d, tnear, tfar, t, u, v)) {
+                const int gid = __float_as_int(t0.w);
+                if (t < best || (t == best && gid < best_gid)) {
+                    best = t; best_gid = gid;
+                    hit.t = t; hit.u = u; hit.v = v; hit.gid = gid;
+                    if (kAny) return true;
+                }
+            }
+        }
+        if (sp == 0) return hit.gid >= 0;
+        node = stack[--sp];
+    }
+}
+
 // Ray setup of rt::Embree::initializeRay (rt/Embree.cpp:107-130) for the
 // segment start -> start + dir * length.
 __device__ __forceinline__ void segment_ray(V3 start, V3 dir, float length, V3& o, V3& d, float& tnear,
@@ -924,6 +988,7 @@ struct SegHit {
 };
 
 // rt::Embree::traceSegment + initializeRay (rt/Embree.cpp:107-177).
+template <bool kWide = false>
 __device__ __forceinline__ void trace_segment(const DevScene& s, V3 start, V3 end, int flags, SegHit& r,
                                               int* overflow) {
     r.hit = false;
@@ -931,7 +996,9 @@ __device__ __forceinline__ void trace_segment(const DevScene& s, V3 start, V3 en
         V3 dir = sub3(end, start);
         float len = normalize3(dir);
         RayHit h;
-        if (!traverse<false>(s, start, dir, 0.01f, len, h, overflow)) return;
+        const bool met = kWide ? traverse4<false>(s, start, dir, 0.01f, len, h)
+                               : traverse<false>(s, start, dir, 0.01f, len, h, overflow);
+        if (!met) return;
         V3 point = add3(start, mul3(dir, h.t));
         int4 f = __ldg(s.tri_vidx + h.gid);
         float4 rgba = make_float4(1.f, 1.f, 1.f, 1.f);
