@@ -531,8 +531,8 @@ extern "C" int rl_trace_segments(const rl_scene* s, int64_t n, const float* d_se
                                  float* d_rgba, float* d_uv, void* stream) {
     if (!s || (n > 0 && (!d_seg || !d_hit))) return fail(RL_INVALID_CALL, "rl_trace_segments: null argument");
     if (n <= 0) return RL_OK;
-    (s->dev.wide && n <= kFewRays ? k_trace_segments<true> : k_trace_segments<false>)
-        <<<blocks_for(n, 128), 128, 0, S(stream)>>>(s->dev, n, d_seg, flags, d_hit, d_t_uv, d_mesh_face, d_point,
+    auto* kern = s->dev.wide && n <= kFewRays ? k_trace_segments<true> : k_trace_segments<false>;
+    kern<<<blocks_for(n, 128), 128, 0, S(stream)>>>(s->dev, n, d_seg, flags, d_hit, d_t_uv, d_mesh_face, d_point,
                                                     d_normal, d_rgba, d_uv, s->d_status);
     CK_LAUNCH("k_trace_segments");
     return RL_OK;

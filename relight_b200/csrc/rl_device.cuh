@@ -992,31 +992,38 @@ template <bool kWide = false>
 __device__ __forceinline__ void trace_segment(const DevScene& s, V3 start, V3 end, int flags, SegHit& r,
                                               int* overflow) {
     r.hit = false;
-    for (int step = 0;; step++) {
-        V3 dir = sub3(end, start);
-        float len = normalize3(dir);
-        RayHit h;
-        const bool met = kWide ? traverse4<false>(s, start, dir, 0.01f, len, h)
-                               : traverse<false>(s, start, dir, 0.01f, len, h, overflow);
-        if (!met) return;
-        V3 point = add3(start, mul3(dir, h.t));
-        int4 f = __ldg(s.tri_vidx + h.gid);
-        float4 rgba = make_float4(1.f, 1.f, 1.f, 1.f);
-        if ((flags & (kHitColor | kHitUseAlpha)) != 0) rgba = face_color(s, f, h.u, h.v);
-        if ((flags & kHitUseAlpha) && rgba.w <= 0.1f && step < 25) {
+    V3 dir = sub3(end, start);
+    float len = normalize3(dir);
+    RayHit h;
+    auto walk = [&] {
+        return kWide ? traverse4<false>(s, start, dir, 0.01f, len, h) : traverse<false>(s, start, dir, 0.01f, len, h, overflow);
+    };
+    if (!walk()) return;
+    V3 point = add3(start, mul3(dir, h.t));
+    int4 f = __ldg(s.tri_vidx + h.gid);
+    float4 rgba = make_float4(1.f, 1.f, 1.f, 1.f);
+    if ((flags & (kHitColor | kHitUseAlpha)) != 0) rgba = face_color(s, f, h.u, h.v);
+    // on through transparent texels.  The first walk is outside the loop: with
+    // all walks in it the lanes of a warp took them apart (1M segments 579 us,
+    // 229 so; textured room, direct light and AO of 384^2, 287 -> 276).
+    if (flags & kHitUseAlpha)
+        for (int step = 0; rgba.w <= 0.1f && step < 25; step++) {
             start = add3(point, dir);
-            continue;
+            dir = sub3(end, start);
+            len = normalize3(dir);
+            if (!walk()) return;
+            point = add3(start, mul3(dir, h.t));
+            f = __ldg(s.tri_vidx + h.gid);
+            rgba = face_color(s, f, h.u, h.v);
         }
-        r.hit = true;
-        r.point = point;
-        r.mesh = f.w;
-        r.face = h.gid - s.mesh_first_tri[f.w];
-        r.t = h.t; r.u = h.u; r.v = h.v;
-        if (flags & kHitNormal) r.normal = interp3(s.nrm, f, h.u, h.v);
-        if (flags & kHitColor) r.rgba = rgba;
-        if (flags & kHitUv) r.uv = interp2(s.uv1, f, h.u, h.v);
-        return;
-    }
+    r.hit = true;
+    r.point = point;
+    r.mesh = f.w;
+    r.face = h.gid - s.mesh_first_tri[f.w];
+    r.t = h.t; r.u = h.u; r.v = h.v;
+    if (flags & kHitNormal) r.normal = interp3(s.nrm, f, h.u, h.v);
+    if (flags & kHitColor) r.rgba = rgba;
+    if (flags & kHitUv) r.uv = interp2(s.uv1, f, h.u, h.v);
 }
 
 // Hit / miss of a segment as the reference sees it (traceSegment's bool).
