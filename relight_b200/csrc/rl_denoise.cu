@@ -861,7 +861,7 @@ __global__ void __launch_bounds__(128, 1) k_conv3x3_wgrad(const __grid_constant_
 // Launch with programmatic stream serialisation (see pdl_wait).
 // Every kernel of a forward pass and of a training step is launched so: the
 // gradients', the loss's and the optimiser's launches made a step of 16 patches
-// of 64 x 64 403 -> 387 us, one of 4 of 32 x 32 430 -> 400.
+// of 64 x 64 411 -> 396 us, one of 4 of 32 x 32 430 -> 400.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -964,13 +964,11 @@ extern "C" int rl_dn_conv3x3(const void* in0, int c0, const void* in1, int c1, i
     a.tap_bytes = (uint32_t)a.nkc_total * (uint32_t)ncols * 16;
     a.wpk = (const bf16*)weights;
     // partial accumulators: four issuers, each in its own 128-column quarter
-    // of tensor memory; two issuers 256 columns apart for 256 columns, and for
-    // 128 where a CTA has several tiles of few MMAs (at most 32 input
-    // channels): two accumulator sets then let the epilogue, the longer part,
-    // overlap the next tile's MMAs (32 -> 64 + 32 channels with masks at
-    // 16 x 64 x 64 pixels: 38.5 -> 25 us)
-    const long long half_tiles = (long long)((width + 7) / 8) * ((height + kHTileH - 1) / kHTileH) * images;
-    a.issuers = a.tmem_cols <= 64 || (a.tmem_cols == 128 && (a.nkc_total > 4 || half_tiles <= 148)) ? 4 : 2;
+    // of tensor memory; two issuers 256 columns apart for 256 columns.  (Two
+    // issuers and two accumulator sets for 128 columns as well made a data
+    // gradient of 32 channels 38 -> 25 us, but add the partial sums in another
+    // order, which flips BF16 roundings that a training run then carries.)
+    a.issuers = a.tmem_cols <= 128 ? 4 : 2;
     a.pstride = 512 / a.issuers;
     // shared memory: the nine taps of weights resident beside at least two
     // halo stages when they fit (units of one K-step, dealt to the issuers);

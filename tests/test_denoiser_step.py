@@ -74,8 +74,8 @@ def test_forward_takes_any_placement(cuda):
 @pytest.mark.parametrize("n,h,w", [(1, 16, 16), (3, 160, 72)])
 def test_masked_gradient_columns(cuda, n, h, w):
     """A data gradient of 32 channels into 128 columns of which 96 are kept, in
-    one tile per CTA and in several (two issuers, two accumulator sets), against
-    FP32; BF16 outputs of sums of 288 products: 2^-8 of the value and 2^-8 of
+    one tile per CTA and in several, against
+    FP64; BF16 outputs of sums of 288 products: 2^-8 of the value and 2^-8 of
     the largest."""
     import torch
     from relight_b200 import denoise as D
