@@ -572,9 +572,9 @@ __global__ void k_intersect_few(DevScene s, long long n, const float4* rays, int
     }
 }
 
-// The same for more rays: a warp takes `rays_per_warp` rays one after another in its lanes: a lane
-// whose ray ended waits until kRayRefill of them have, then they start
-// together, and leaves wait for each other in the same way.
+// The same for more rays: a warp takes `rays_per_warp` of them one after another
+// in its lanes: a lane whose ray ended waits until kRayRefill of them have, then
+// they start together, and leaves wait for each other in the same way.
 constexpr int kRayRefill = 8, kRayThreads = 64;
 
 template <bool kAny, bool kPacked>
